@@ -9,6 +9,7 @@
 
 #include "gen.cuh"
 #include "internal.h"
+#include "rows.cuh"
 #include "spmspv.h"
 
 namespace sfci {
@@ -59,6 +60,7 @@ void scratch_free_all(Ctx& c) {
   for (auto& kv : c.scratch)
     if (kv.second.p) cudaFree(kv.second.p);
   c.scratch.clear();
+  rows_free(c);
 }
 
 void scratch_release(Ctx& c, const char* name) {

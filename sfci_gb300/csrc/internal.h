@@ -44,6 +44,9 @@ struct Ctx {
   HamHost ham;
   double* d_h1 = nullptr;
   double* d_V = nullptr;
+  // row-driven products (rows.cu): oriented opposite-spin integrals, binomials
+  double* d_row_os = nullptr;  // and the directed integrals of the singles after them
+  unsigned* d_row_bin = nullptr;
   cudaStream_t stream = nullptr;
   int sm_count = 0;
   std::map<std::string, Buf> scratch;

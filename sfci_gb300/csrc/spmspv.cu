@@ -30,8 +30,10 @@
 #include <vector>
 
 #include "gen.cuh"
+#include "merge.cuh"
 #include "prims.cuh"
 #include "plan.h"
+#include "rows.cuh"
 #include "screen.cuh"
 #include "spmspv.h"
 #include "table.cuh"
@@ -59,6 +61,7 @@ constexpr int RUN_CAP = 2048;  // class passes: (occupied pair, class block) run
 constexpr double LEAF_TERMS = 1024.0;                 // terms a leaf is sized for (at most, on average)
 
 enum { M_COUNT = 0, M_SCATTER = 1, M_ENERGY = 2, M_PROJECT = 3, M_LABEL = 4 };
+constexpr u64 ROWS_MIN_TERMS = 1ull << 20;  // below it rows_product never pays (rows.cu has the rule)
 constexpr int PROJ_MAX = 64;  // vectors of one projection sweep
 
 template <int W> struct PartIPT;
@@ -107,61 +110,6 @@ __device__ __forceinline__ unsigned leaf_slot(const u64& k, int tbits) {
 }
 __device__ __forceinline__ unsigned leaf_slot(const K128& k, int tbits) {
   return (unsigned)(((k.lo * 0xd6e8feb86659fd93ull) ^ (k.hi * 0x94d049bb133111ebull)) >> (64 - tbits));
-}
-
-// The post-merge cut |a| > cut as an integer test on the accumulated sum: sums
-// whose magnitude is at most `below` (cut * 2^FX_FRAC * (1 - 2^-40), rounded
-// down) cannot survive and are dropped without converting them; the rest are
-// converted and compared exactly.  A negative cut keeps everything.
-struct FxCut {
-  u64 below_lo, below_hi;
-  long long cutk;  // cut_key(cut)
-  int all;
-};
-// the cut on a 128-bit sum (hi:lo) in units of 2^-FX_FRAC
-__device__ __forceinline__ bool fx_survives_value(u64 lo, u64 hi, const FxCut& c, double& v) {
-  if (!c.all) {
-    u64 mlo = lo, mhi = hi;
-    if ((long long)hi < 0) {
-      mhi = ~hi + (lo == 0 ? 1ull : 0ull);
-      mlo = 0ull - lo;
-    }
-    if (mhi < c.below_hi || (mhi == c.below_hi && mlo <= c.below_lo)) return false;
-  }
-  v = fx_to_double(lo, hi);
-  return above_cut(v, c.cutk);
-}
-// the cut on a split accumulator (acc_hi * 2^FX_SPLIT + acc_lo)
-__device__ __forceinline__ bool fx_survives(u64 acc_lo, u64 acc_hi, const FxCut& c, double& v) {
-  u64 lo, hi;
-  fx_value(acc_lo, acc_hi, lo, hi);
-  return fx_survives_value(lo, hi, c, v);
-}
-static FxCut fx_cut(double cut) {
-  FxCut c{};
-  c.cutk = cut_key(cut);
-  c.all = cut < 0.0 ? 1 : 0;
-  if (!c.all) {
-    // cut * 2^FX_FRAC is exact in double; the 2^-40 margin covers the rounding
-    // of the product below and of the final conversion
-    const double y = std::ldexp(cut, FX_FRAC) * (1.0 - std::ldexp(1.0, -40));
-    const unsigned __int128 t = y >= std::ldexp(1.0, 127) ? ~(unsigned __int128)0 >> 1 : (unsigned __int128)y;
-    c.below_lo = (u64)t;
-    c.below_hi = (u64)(t >> 64);
-  }
-  return c;
-}
-
-// add x exactly to a 128-bit fixed-point accumulator acc[0..1] (low, high):
-// the carry of each low-word addition is known from its returned old value, so
-// the total is the exact sum whatever the order of the additions
-__device__ __forceinline__ void fx_atomic_add128(u64* acc, double x, unsigned& bad) {
-  u64 l, h;
-  fx128_of(x, l, h, bad);
-  if ((l | h) == 0) return;
-  const u64 old = atomicAdd((unsigned long long*)acc, (unsigned long long)l);
-  const u64 hh = h + ((old + l < old) ? 1ull : 0ull);
-  if (hh) atomicAdd((unsigned long long*)(acc + 1), (unsigned long long)hh);
 }
 
 // add a term's two addends to an accumulator (results unused: reductions)
@@ -1605,11 +1553,11 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
       ng = ns + nx;
     }
   }
+  u64 conn = 0;  // terms of a determinant, the most its spin counts allow
   {
     // a merged determinant receives at most one term per input determinant
     // connected to it, i.e. at most the term count of a determinant with its
     // spin occupations; the merge accumulators are exact up to FX_MAX_TERMS
-    u64 conn = 0;
     for (int a0 = 0; a0 <= c.ne; ++a0) {
       const int a1 = c.ne - a0;
       if (a0 > c.M || a1 > c.M) continue;
@@ -1617,6 +1565,37 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
     }
     if (std::min<u64>(conn, ns) > FX_MAX_TERMS)
       return set_error(SFCI_ERR_UNSUPPORTED, "SpMSpV: determinants connect to more than 2^19 others");
+  }
+  // Row-driven form: whole products on one plain Hamiltonian.  The partitioned
+  // pipeline below takes the rest (extra sources, screens, batches), the plans a
+  // caller asked for by a device budget or by class passes, and what
+  // rows_product declines.
+  if (ng == ns && !c.screen && !c.ninst && !c.opts.mem_budget && c.tune_class_passes <= 0 &&
+      ns * conn >= ROWS_MIN_TERMS) {
+    RowsResult<W> rr;
+    bool done = false;
+    phase_end(c, tok);
+    if ((st = rows_product<W>(c, src_k, src_a, ns, lambda, coeff, out.cap, &rr, &done))) return st;
+    if (done) {
+      c.stats[1] = rr.terms;
+      c.stats[2] = rr.uniq;
+      c.stats[3] = rr.nsurv;
+      c.stats[5] = 1;
+      c.stats[6] = rr.units;
+      c.last_pruned = rr.pruned;
+      if (rr.uniq) c.dup_est = (double)rr.terms / (double)rr.uniq;
+      *diag = fx_to_double(rr.dexact[0], rr.dexact[1]);
+      size_t m = 0;
+      tok = phase_begin(c, rr.nsurv > out.cap ? PH_SELECT : PH_SORT);
+      if ((st = select_sorted<W>(c, rr.sk, rr.sa, rr.nsurv, out.cap, &m))) return st;
+      SFCI_CUDA(cudaMemcpyAsync(out.keys, rr.sk, m * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
+      SFCI_CUDA(cudaMemcpyAsync(out.amps, rr.sa, m * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+      phase_end(c, tok);
+      out.len = m;
+      c.stats[4] = m;
+      return SFCI_OK;
+    }
+    tok = phase_begin(c, PH_OTHER);
   }
   // learned screen: the kept term groups of each source.  Products with extra
   // single-term sources (the linear solver's) stay unscreened.
