@@ -33,6 +33,7 @@
 #include "merge.cuh"
 #include "prims.cuh"
 #include "plan.h"
+#include "pairs.cuh"
 #include "rows.cuh"
 #include "screen.cuh"
 #include "spmspv.h"
@@ -61,6 +62,11 @@ constexpr int RUN_CAP = 2048;  // class passes: (occupied pair, class block) run
 constexpr double LEAF_TERMS = 1024.0;                 // terms a leaf is sized for (at most, on average)
 
 enum { M_COUNT = 0, M_SCATTER = 1, M_ENERGY = 2, M_PROJECT = 3, M_LABEL = 4 };
+// terms of a full sweep from which the pair search (pairs.cu) is used: its fixed
+// part is some twenty launches, 140 us at 300 sources of 20 spin orbitals (2.6e5
+// terms) against 109 for the sweep, 157 against 159 at 1,000, 173 against 522 at 64
+// of 56 spin orbitals
+constexpr u64 PAIRS_MIN_TERMS = 1ull << 20;
 constexpr u64 ROWS_MIN_TERMS = 1ull << 20;  // below it rows_product never pays (rows.cu has the rule)
 constexpr int PROJ_MAX = 64;  // vectors of one projection sweep
 
@@ -1495,6 +1501,17 @@ __global__ void k_scaled_copy(double* __restrict__ dst, const double* __restrict
     dst[i] = a * src[i];
 }
 
+// terms of a determinant, the most any split of the electrons over the spins gives
+static u64 most_terms(const Ctx& c) {
+  u64 conn = 0;
+  for (int a0 = 0; a0 <= c.ne; ++a0) {
+    const int a1 = c.ne - a0;
+    if (a0 > c.M || a1 > c.M) continue;
+    conn = std::max<u64>(conn, det_terms(a0, c.M - a0, a1, c.M - a1));
+  }
+  return conn;
+}
+
 template <int W>
 int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, double* diag, const SpExtra* ex) {
   typedef typename KeyOf<W>::T KT;
@@ -1553,16 +1570,11 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
       ng = ns + nx;
     }
   }
-  u64 conn = 0;  // terms of a determinant, the most its spin counts allow
+  const u64 conn = most_terms(c);
   {
     // a merged determinant receives at most one term per input determinant
     // connected to it, i.e. at most the term count of a determinant with its
     // spin occupations; the merge accumulators are exact up to FX_MAX_TERMS
-    for (int a0 = 0; a0 <= c.ne; ++a0) {
-      const int a1 = c.ne - a0;
-      if (a0 > c.M || a1 > c.M) continue;
-      conn = std::max<u64>(conn, det_terms(a0, c.M - a0, a1, c.M - a1));
-    }
     if (std::min<u64>(conn, ns) > FX_MAX_TERMS)
       return set_error(SFCI_ERR_UNSUPPORTED, "SpMSpV: determinants connect to more than 2^19 others");
   }
@@ -2111,6 +2123,16 @@ int energy_impl(Ctx& c, const Vec& psi, double* E) {
   int st;
   u64 *doff = nullptr, T = 0;
   double* diagE = nullptr;
+  if (!c.ninst && psi.len * most_terms(c) >= PAIRS_MIN_TERMS) {
+    bool done = false;
+    if ((st = pairs_energy<W>(c, (const KT*)psi.keys, psi.amps, psi.len, E, &T, &done))) return st;
+    if (done) {
+      for (auto& s : c.stats) s = 0;
+      c.stats[0] = psi.len;
+      c.stats[1] = T;
+      return SFCI_OK;
+    }
+  }
   if ((st = prep_dets<W>(c, (const KT*)psi.keys, psi.len, &doff, &diagE, &T))) return st;
   for (auto& s : c.stats) s = 0;
   c.stats[0] = psi.len;
@@ -2229,27 +2251,34 @@ int project_impl(Ctx& c, const Vec& src, double lambda, const Vec* const* basis,
     SFCI_LAUNCH(c, k_key_insert<KT>, gr, 256, 0, (const KT*)basis[j]->keys, l, tk, (unsigned)(tsz - 1));
   }
   int st;
-  u64 *doff = nullptr, T = 0;
-  double* diagE = nullptr;
-  if ((st = prep_dets<W>(c, (const KT*)src.keys, src.len, &doff, &diagE, &T))) return st;
-  const unsigned G = gen_grid(c, T);
-  GenArgs<KT> g{};
-  g.keys = (const KT*)src.keys;
-  g.amps = src.amps;
-  g.ndet = src.len;
-  g.doff = doff;
-  g.diagE = diagE;
-  g.coeff = 1.0;
-  g.lambda = lambda;
-  g.h = ham_view(c);
-  g.T = T;
-  g.b1 = 1;
-  g.tkeys = tk;
-  g.tmask = (unsigned)(tsz - 1);
-  g.plo = plo;
-  g.phi = phi;
-  g.pbad = bad;
-  if ((st = launch_gen<W, M_PROJECT>(c, g, G, 0))) return st;
+  bool done = false;
+  if (!c.ninst && src.len * most_terms(c) >= PAIRS_MIN_TERMS) {
+    if ((st = pairs_project<W>(c, (const KT*)src.keys, src.amps, src.len, lambda, tk, tsz, plo, phi, &done))) return st;
+    if (!done) SFCI_CUDA(cudaMemsetAsync(acc, 0, (2 * tsz + 1) * sizeof(u64), c.stream));
+  }
+  if (!done) {
+    u64 *doff = nullptr, T = 0;
+    double* diagE = nullptr;
+    if ((st = prep_dets<W>(c, (const KT*)src.keys, src.len, &doff, &diagE, &T))) return st;
+    const unsigned G = gen_grid(c, T);
+    GenArgs<KT> g{};
+    g.keys = (const KT*)src.keys;
+    g.amps = src.amps;
+    g.ndet = src.len;
+    g.doff = doff;
+    g.diagE = diagE;
+    g.coeff = 1.0;
+    g.lambda = lambda;
+    g.h = ham_view(c);
+    g.T = T;
+    g.b1 = 1;
+    g.tkeys = tk;
+    g.tmask = (unsigned)(tsz - 1);
+    g.plo = plo;
+    g.phi = phi;
+    g.pbad = bad;
+    if ((st = launch_gen<W, M_PROJECT>(c, g, G, 0))) return st;
+  }
   unsigned hbad = 0;
   if ((st = read_words(c, bad, sizeof(unsigned), &hbad))) return st;
   if (hbad)
