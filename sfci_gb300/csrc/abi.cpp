@@ -92,18 +92,37 @@ u64* pinned_words(Ctx& c, size_t n) {
   return c.h_pin;
 }
 
+unsigned* coop_error_word(Ctx& c) {
+  if (!c.h_coop) {
+    if (cudaMallocHost(&c.h_coop, sizeof(unsigned)) != cudaSuccess) {
+      cudaGetLastError();
+      c.h_coop = nullptr;
+      set_error(SFCI_ERR_NOMEM, "pinned host word");
+      return nullptr;
+    }
+    *c.h_coop = 0;
+  }
+  return c.h_coop;
+}
+// after a synchronisation: did a grid barrier of the work before it time out?
+static int coop_check(Ctx& c) {
+  if (!c.h_coop || !*(volatile unsigned*)c.h_coop) return SFCI_OK;
+  *c.h_coop = 0;
+  return set_error(SFCI_ERR_CUDA, "grid barrier timed out: the preceding sort or selection is incomplete");
+}
+
 int read_words(Ctx& c, const void* dptr, size_t nbytes, void* host) {
   size_t words = (nbytes + 7) / 8;
   u64* pin = pinned_words(c, words);
   if (!pin) {
     SFCI_CUDA(cudaMemcpyAsync(host, dptr, nbytes, cudaMemcpyDeviceToHost, c.stream));
     SFCI_CUDA(cudaStreamSynchronize(c.stream));
-    return SFCI_OK;
+    return coop_check(c);
   }
   SFCI_CUDA(cudaMemcpyAsync(pin, dptr, nbytes, cudaMemcpyDeviceToHost, c.stream));
   SFCI_CUDA(cudaStreamSynchronize(c.stream));
   memcpy(host, pin, nbytes);
-  return SFCI_OK;
+  return coop_check(c);
 }
 
 // ---- phase timing ----------------------------------------------------------
@@ -254,6 +273,7 @@ int sfci_ctx_create(const char* in_path, int num_orb, int num_e, const sfci_opts
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) coop_error_word(c);  // (made now: pinning a word in the first sort would take longer than the sort)
   if (e == cudaSuccess) e = cudaMalloc(&c.d_h1, c.ham.h1.size() * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&c.d_V, c.ham.V.size() * sizeof(double));
   if (e == cudaSuccess)
@@ -313,6 +333,7 @@ int sfci_batch_create(int n, const char* const* in_paths, const int* num_orb, co
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) coop_error_word(c);  // (made now: pinning a word in the first sort would take longer than the sort)
   std::vector<HamView> views(n);
   c.inst_h1.assign(n, nullptr);
   c.inst_V.assign(n, nullptr);
@@ -473,6 +494,7 @@ int sfci_ctx_destroy(sfci_ctx* x) {
     cudaEventDestroy(p.second.first);
     cudaEventDestroy(p.second.second);
   }
+  if (c.h_coop) cudaFreeHost(c.h_coop);
   if (c.h_pin) cudaFreeHost(c.h_pin);
   if (c.stream) cudaStreamDestroy(c.stream);
   delete x;
@@ -636,7 +658,7 @@ int sfci_vec_download(const sfci_vec* v, uint64_t* keys, double* amps, uint64_t 
   }
   SFCI_CUDA(cudaStreamSynchronize(c.stream));
   if (len) *len = v->v.len;
-  return SFCI_OK;
+  return coop_check(c);
 }
 
 int sfci_vec_copy(sfci_vec* dst, const sfci_vec* src) {

@@ -66,6 +66,7 @@ struct Ctx {
   // pinned host staging for small readbacks
   u64* h_pin = nullptr;
   size_t h_pin_words = 0;
+  unsigned* h_coop = nullptr;  // set by a kernel whose grid barrier ran out of its poll limit
   // batched contexts: one Hamiltonian per instance (device HamView table);
   // ninst = 0 for an ordinary context
   int ninst = 0;

@@ -155,11 +155,213 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const KT* __restrict_
   }
 }
 
+// ---- one launch for vectors of up to COOP_MAX entries ---------------------------
+// The multi-launch passes above cost five launches a digit, whatever the length.
+// Here one cooperative kernel runs every pass: each CTA owns a slice of the input
+// and counts it by digit per warp, publishes its counts, and after a grid barrier
+// adds up the counts of the slices before it, so a pass needs two barriers.  Bound
+// by the latency of its phases (about 17 us a pass at 500,000 entries, of which
+// the barriers take 4).  Measured for 56-bit keys, us, launches -> one kernel: 860
+// entries 162 -> 30, 50,000 213 -> 67, 500,000 288 -> 119, 2,000,000 533 -> 254,
+// 4,000,000 945 -> 655; 68-bit keys 500,000 391 -> 177.  Digits of 8, 9 and 10 bits
+// are within 10% of one another.
+constexpr size_t COOP_MAX = 1u << 22;
+constexpr int CO_THREADS = 1024;
+constexpr int CO_WARPS = CO_THREADS / 32;
+constexpr int CO_DIGIT = 8;
+constexpr int CO_BATCH = 2;  // entries a lane loads ahead
+
+// Grid barrier of a cooperative launch (every CTA is resident): true when all
+// CTAs arrived, false (and *err set) when they did not within the poll limit.
+__device__ bool coop_barrier(unsigned* bar, unsigned target, unsigned* err) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    int ok = 0;
+    for (unsigned spin = 0; spin < (1u << 22); ++spin) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if (v >= target) {
+        ok = 1;
+        break;
+      }
+    }
+    if (!ok) *(volatile unsigned*)err = 1u;
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  const bool ok = s_ok != 0;
+  __syncthreads();
+  return ok;
+}
+
+__device__ __forceinline__ unsigned key_bits(const u64& k, int shift, unsigned mask) { return (unsigned)(k >> shift) & mask; }
+__device__ __forceinline__ unsigned key_bits(const K128& k, int shift, unsigned mask) {
+  if (shift >= 64) return (unsigned)(k.hi >> (shift - 64)) & mask;
+  return (unsigned)((k.lo >> shift) | (shift ? k.hi << (64 - shift) : 0ull)) & mask;
+}
+__device__ __forceinline__ u64 ld_key(const u64* p) { return __ldcg(p); }
+__device__ __forceinline__ K128 ld_key(const K128* p) {
+  K128 k;
+  k.lo = __ldcg((const u64*)p);
+  k.hi = __ldcg((const u64*)p + 1);
+  return k;
+}
+
+// (values written by other CTAs in an earlier pass are read through L2)
+template <class KT>
+__global__ void __launch_bounds__(CO_THREADS, 1) k_rs_coop(KT* ka, double* va, KT* kb, double* vb, unsigned n,
+                                                        unsigned slice, int passes, int bits, uint32_t* cnt,
+                                                        unsigned* bar, unsigned* err) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const unsigned nd = 1u << bits, mask = nd - 1u, G = gridDim.x, b = blockIdx.x;
+  uint32_t* whist = reinterpret_cast<uint32_t*>(smem);  // [CO_WARPS][nd]
+  uint32_t* base = whist + CO_WARPS * nd;               // [nd]
+  __shared__ uint32_t s_scan[CO_WARPS + 1];
+  __shared__ uint32_t s_bef[CO_THREADS], s_tot[CO_THREADS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u, ws = slice / CO_WARPS;  // a multiple of 32
+  const unsigned w0 = min(n, b * slice + warp * ws), w1 = min(n, w0 + ws);
+  uint32_t* wh = whist + warp * nd;
+  unsigned target = 0;
+  for (int p = 0; p < passes; ++p) {
+    const int shift = p * bits;
+    for (unsigned d = tid; d < CO_WARPS * nd; d += CO_THREADS) whist[d] = 0;
+    __syncthreads();
+    for (unsigned i = w0 + lane; i < w1; i += 32) atomicAdd(&wh[key_bits(ld_key(ka + i), shift, mask)], 1u);
+    __syncthreads();
+    // counts of the slice; each warp's become its offset within the slice
+    uint32_t mine = 0;
+    if (tid < (int)nd) {
+#pragma unroll 8
+      for (int w = 0; w < CO_WARPS; ++w) {
+        const uint32_t t = whist[w * nd + tid];
+        whist[w * nd + tid] = mine;
+        mine += t;
+      }
+    }
+    uint32_t before = 0, total = mine;
+    if (G > 1) {
+      uint32_t* c = cnt + (size_t)(p & 1) * G * nd;  // the previous pass's counts may still be read
+      if (tid < (int)nd) __stcg(c + (size_t)b * nd + tid, mine);
+      target += G;
+      if (!coop_barrier(bar, target, err)) return;
+      // thread (part, digit) adds its share of the slices; the parts meet in shared memory
+      const unsigned d = tid & mask, part = tid >> bits, parts = CO_THREADS >> bits;
+      uint32_t bef = 0, tot = 0;
+      for (unsigned q = part; q < G; q += 8 * parts) {
+        uint32_t v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = q + u * parts < G ? __ldcg(c + (size_t)(q + u * parts) * nd + d) : 0u;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (q + u * parts < b) bef += v[u];
+          tot += v[u];
+        }
+      }
+      s_bef[tid] = bef;
+      s_tot[tid] = tot;
+      __syncthreads();
+      if (tid < (int)nd) {
+        total = 0;
+        for (unsigned q = 0; q < parts; ++q) {
+          before += s_bef[q * nd + tid];
+          total += s_tot[q * nd + tid];
+        }
+      }
+    }
+    const uint32_t ex = block_excl_scan<uint32_t, CO_THREADS>(tid < (int)nd ? total : 0u, nullptr, s_scan);
+    if (tid < (int)nd) base[tid] = ex + before;
+    __syncthreads();
+    for (unsigned i0 = w0; i0 < w1; i0 += 32 * CO_BATCH) {
+      KT k[CO_BATCH];
+      double v[CO_BATCH];
+#pragma unroll
+      for (int q = 0; q < CO_BATCH; ++q) {
+        const unsigned i = i0 + q * 32 + lane;
+        if (i < w1) {
+          k[q] = ld_key(ka + i);
+          v[q] = __ldcg(va + i);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < CO_BATCH; ++q) {
+        if (i0 + q * 32 >= w1) break;  // (the same for the whole warp)
+        const bool ok = i0 + q * 32 + lane < w1;
+        const unsigned d = ok ? key_bits(k[q], shift, mask) : nd + lane;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        uint32_t pos = 0;
+        if (ok) pos = wh[d] + __popc(peers & lt);
+        __syncwarp();
+        if (ok) {
+          if (lane == __ffs(peers) - 1) wh[d] += __popc(peers);
+          pos += base[d];
+          kb[pos] = k[q];
+          vb[pos] = v[q];
+        }
+        __syncwarp();
+      }
+    }
+    if (G > 1) {
+      target += G;
+      if (!coop_barrier(bar, target, err)) return;
+    } else {
+      __syncthreads();
+    }
+    KT* tk = ka;
+    ka = kb;
+    kb = tk;
+    double* tv = va;
+    va = vb;
+    vb = tv;
+  }
+  if (passes & 1)  // the result is in the second buffers
+    for (unsigned i = w0 + lane; i < w1; i += 32) {
+      kb[i] = ld_key(ka + i);
+      vb[i] = __ldcg(va + i);
+    }
+}
+
+// entries a CTA takes, for n entries
+static unsigned coop_slice(const Ctx& c, size_t n) {
+  const size_t s = (n + c.sm_count - 1) / c.sm_count;
+  return (unsigned)std::max<size_t>(1024, (s + 1023) / 1024 * 1024);
+}
+
+template <int W>
+static int radix_sort_coop(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, int nbits) {
+  typedef typename KeyOf<W>::T KT;
+  const int nb8 = (nbits + 7) / 8 * 8;  // the bits the 8-bit passes cover
+  int passes = (nb8 + CO_DIGIT - 1) / CO_DIGIT, bits = (nb8 + passes - 1) / passes;
+  unsigned slice = coop_slice(c, n), un = (unsigned)n;
+  const unsigned G = (un + slice - 1) / slice;
+  KT* k2 = (KT*)scratch_get(c, "rs_keys", n * sizeof(KT));
+  double* v2 = (double*)scratch_get(c, "rs_vals", n * sizeof(double));
+  uint32_t* cnt = (uint32_t*)scratch_get(c, "rs_coop", (4 + 2 * ((size_t)c.sm_count << CO_DIGIT)) * sizeof(uint32_t));
+  if (!k2 || !v2 || !cnt) return SFCI_ERR_NOMEM;
+  unsigned* bar = cnt;
+  uint32_t* cm = cnt + 4;
+  unsigned* err = coop_error_word(c);
+  if (!err) return SFCI_ERR_NOMEM;
+  if (G > 1) SFCI_CUDA(cudaMemsetAsync(bar, 0, sizeof(unsigned), c.stream));
+  const size_t sm = sizeof(uint32_t) * ((size_t)(CO_WARPS + 1) << bits);
+  SFCI_CUDA(cudaFuncSetAttribute(k_rs_coop<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(uint32_t) * ((size_t)(CO_WARPS + 1) << CO_DIGIT))));
+  void* args[] = {&keys, &vals, &k2, &v2, &un, &slice, &passes, &bits, &cm, &bar, &err};
+  SFCI_CUDA(cudaLaunchCooperativeKernel((const void*)k_rs_coop<KT>, dim3(G), dim3(CO_THREADS), args, sm, c.stream));
+  c.launches++;
+  return SFCI_OK;
+}
+
 template <int W>
 int radix_sort_pairs(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, int nbits) {
   typedef typename KeyOf<W>::T KT;
   if (n <= 1 || nbits <= 0) return SFCI_OK;
   if (n >= (1ull << 32)) return set_error(SFCI_ERR_UNSUPPORTED, "radix sort beyond 2^32 items");
+  if (n <= COOP_MAX) return radix_sort_coop<W>(c, keys, vals, n, nbits);
   size_t ntiles = (n + RS_TILE - 1) / RS_TILE;
   KT* k2 = (KT*)scratch_get(c, "rs_keys", n * sizeof(KT));
   double* v2 = (double*)scratch_get(c, "rs_vals", n * sizeof(double));
@@ -407,6 +609,208 @@ static int compact_rule(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia
   return SFCI_OK;
 }
 
+// ---- selection and compaction in one launch (up to COOP_MAX entries) ---------------
+// The launches above read a histogram back after each of six digits and the
+// counts after that: eight round trips to the host.  Here the digits, the counts
+// and the compaction are one cooperative kernel with a grid barrier in place of
+// each round trip: the top 400,000 of 1,400,000 entries take 64 us (270 before),
+// of 17,000 38 us (200).  A digit whose bin is taken whole ends the search: the
+// threshold is then the bin's lower edge and no tie has to be ranked.
+struct SelArgs {
+  const double* a;
+  unsigned n, slice;
+  int mode;            // 0: keep |a| above lb only; 1: the k largest first
+  u64 k;
+  long long low_key;   // keep bits above this as well (-1: everything)
+  uint32_t* hist;      // [6][4096], zero
+  uint32_t* cnt;       // [2][G]
+  unsigned *bar, *err;
+  u64* m;              // entries kept
+};
+constexpr int SEL_COPIES = 4;
+
+template <class KT>
+__global__ void __launch_bounds__(CO_THREADS, 1) k_sel_coop(SelArgs s, const KT* __restrict__ ik, KT* __restrict__ ok,
+                                                         double* __restrict__ oa) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint32_t* sh = reinterpret_cast<uint32_t*>(smem);  // [SEL_COPIES][4096] (mode 1)
+  __shared__ uint32_t s_scan[CO_WARPS + 1];
+  __shared__ uint32_t s_g[CO_WARPS], s_e[CO_WARPS];
+  __shared__ unsigned s_bin, s_acc, s_cnt;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned G = gridDim.x, b = blockIdx.x, ws = s.slice / CO_WARPS;
+  const unsigned w0 = min(s.n, b * s.slice + warp * ws), w1 = min(s.n, w0 + ws);
+  unsigned target = 0;
+  u64 lb = 0, tau = ~0ull, need_eq = 0;  // keep bits >= lb, and need_eq of those equal to tau
+  if (s.mode == 1) {
+    const int shifts[6] = {51, 39, 27, 15, 3, 0}, widths[6] = {12, 12, 12, 12, 12, 3};
+    u64 prefix = 0, need = s.k;
+    bool whole = false;
+    int r = 0;
+    for (; r < 6 && !whole; ++r) {
+      const unsigned nb = 1u << widths[r];
+      const int shift = shifts[r], pshift = shift + widths[r];
+      for (unsigned i = tid; i < SEL_COPIES * 4096; i += CO_THREADS) sh[i] = 0;
+      __syncthreads();
+      uint32_t* h = sh + (warp & (SEL_COPIES - 1)) * 4096;
+      for (unsigned i = w0 + lane; i < w1; i += 32) {
+        const u64 x = abs_bits(s.a[i]);
+        if (r == 0 || (x >> pshift) == prefix) atomicAdd(&h[(unsigned)(x >> shift) & (nb - 1u)], 1u);
+      }
+      __syncthreads();
+      uint32_t* gh = s.hist + r * 4096;
+      for (unsigned i = tid; i < nb; i += CO_THREADS) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int q = 0; q < SEL_COPIES; ++q) v += sh[q * 4096 + i];
+        if (v) atomicAdd(gh + i, v);
+      }
+      target += G;
+      if (!coop_barrier(s.bar, target, s.err)) return;
+      // the bin that holds the need-th largest: thread t looks at bins from the top
+      uint32_t v[4], sum = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned i = tid * 4 + q;  // i-th bin from the top
+        v[q] = i < nb ? __ldcg(gh + (nb - 1u - i)) : 0u;
+        sum += v[q];
+      }
+      uint32_t acc = block_excl_scan<uint32_t, CO_THREADS>(sum, nullptr, s_scan);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (acc < need && need <= (u64)acc + v[q]) {
+          s_bin = nb - 1u - (tid * 4 + q);
+          s_acc = acc;
+          s_cnt = v[q];
+        }
+        acc += v[q];
+      }
+      __syncthreads();
+      need -= s_acc;
+      prefix = (prefix << widths[r]) | s_bin;
+      whole = s_cnt == need;
+      if (whole) lb = prefix << shift;
+      __syncthreads();
+    }
+    if (!whole) {
+      tau = prefix;
+      lb = tau + 1;
+      need_eq = need;
+    }
+  }
+  const u64 low = (u64)(s.low_key + 1);
+  if (lb < low) lb = low;
+  if (need_eq && tau < low) need_eq = 0;
+  // counts: kept outright, ties
+  uint32_t g = 0, e = 0;
+  for (unsigned i0 = w0; i0 < w1; i0 += 32) {
+    const u64 x = i0 + lane < w1 ? abs_bits(s.a[i0 + lane]) : 0ull;
+    const bool in = i0 + lane < w1;
+    g += __popc(__ballot_sync(0xffffffffu, in && x >= lb));
+    e += __popc(__ballot_sync(0xffffffffu, in && need_eq && x == tau));
+  }
+  if (lane == 0) {
+    s_g[warp] = g;
+    s_e[warp] = e;
+  }
+  __syncthreads();
+  u64 gr = 0, er = 0, gtot = 0, etot = 0;  // before this warp; over all
+  {
+    uint32_t cg = 0, ce = 0;
+    for (int w = 0; w < CO_WARPS; ++w) {
+      if (w == warp) {
+        gr = cg;
+        er = ce;
+      }
+      cg += s_g[w];
+      ce += s_e[w];
+    }
+    gtot = cg;
+    etot = ce;
+    if (G > 1) {
+      if (tid == 0) {
+        __stcg(s.cnt + 2 * b, cg);
+        __stcg(s.cnt + 2 * b + 1, ce);
+      }
+      target += G;
+      if (!coop_barrier(s.bar, target, s.err)) return;
+      u64 bg = 0, be = 0;
+      gtot = etot = 0;
+      for (unsigned q = lane; q < G; q += 32) {
+        const u64 x = __ldcg(s.cnt + 2 * q), y = __ldcg(s.cnt + 2 * q + 1);
+        if (q < b) {
+          bg += x;
+          be += y;
+        }
+        gtot += x;
+        etot += y;
+      }
+      bg = warp_sum(bg);
+      be = warp_sum(be);
+      gtot = warp_sum(gtot);
+      etot = warp_sum(etot);
+      gr += bg;
+      er += be;
+    }
+  }
+  // of the ties, the last need_eq are kept
+  const u64 skip = etot > need_eq ? etot - need_eq : 0ull;
+  if (b == 0 && tid == 0) *s.m = gtot + (etot - skip);
+  const unsigned lt = (1u << lane) - 1u;
+  for (unsigned i0 = w0; i0 < w1; i0 += 32) {
+    const unsigned i = i0 + lane;
+    const bool in = i < w1;
+    const double v = in ? s.a[i] : 0.0;
+    const u64 x = abs_bits(v);
+    const bool kg = in && x >= lb, ke = in && need_eq && x == tau;
+    const unsigned mg = __ballot_sync(0xffffffffu, kg), me = __ballot_sync(0xffffffffu, ke);
+    const u64 el = er + __popc(me & lt);
+    if (kg || (ke && el >= skip)) {
+      const u64 pos = gr + __popc(mg & lt) + (el > skip ? el - skip : 0ull);
+      ok[pos] = ik[i];
+      oa[pos] = v;
+    }
+    gr += __popc(mg);
+    er += __popc(me);
+  }
+}
+
+// mode 0: entries with bits above low_key; mode 1: the k largest first (0 < k < n)
+template <int W>
+static int select_coop(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, int mode, size_t k,
+                       long long low_key, typename KeyOf<W>::T* ok, double* oa, size_t* m) {
+  typedef typename KeyOf<W>::T KT;
+  const size_t words = 6 * 4096 + 2 * (size_t)c.sm_count + 8;
+  uint32_t* buf = (uint32_t*)scratch_get(c, "sel_coop", words * sizeof(uint32_t));
+  unsigned* err = coop_error_word(c);
+  if (!buf || !err) return SFCI_ERR_NOMEM;
+  SelArgs s{};
+  s.a = ia;
+  s.n = (unsigned)n;
+  s.slice = coop_slice(c, n);
+  s.mode = mode;
+  s.k = k;
+  s.low_key = low_key;
+  s.m = (u64*)buf;
+  s.bar = buf + 2;
+  s.hist = buf + 4;
+  s.cnt = buf + 4 + 6 * 4096;
+  s.err = err;
+  const unsigned G = (unsigned)((n + s.slice - 1) / s.slice);
+  SFCI_CUDA(cudaMemsetAsync(buf, 0, (mode == 1 ? 4 + 6 * 4096 : 4) * sizeof(uint32_t), c.stream));
+  const size_t sm = mode == 1 ? SEL_COPIES * 4096 * sizeof(uint32_t) : 0;
+  SFCI_CUDA(cudaFuncSetAttribute(k_sel_coop<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(SEL_COPIES * 4096 * sizeof(uint32_t))));
+  void* args[] = {&s, &ik, &ok, &oa};
+  SFCI_CUDA(cudaLaunchCooperativeKernel((const void*)k_sel_coop<KT>, dim3(G), dim3(CO_THREADS), args, sm, c.stream));
+  c.launches++;
+  u64 got = 0;
+  int st = read_words(c, s.m, sizeof(u64), &got);
+  if (st) return st;
+  *m = (size_t)got;
+  return SFCI_OK;
+}
+
 template <int W>
 int compact_top(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, u64 tau, size_t need_eq,
                 double tiny, typename KeyOf<W>::T* ok, double* oa, size_t* m) {
@@ -417,6 +821,7 @@ int compact_top(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t
 template <int W>
 int compact_cut(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, double cut,
                 typename KeyOf<W>::T* ok, double* oa, size_t* m) {
+  if (n && n <= COOP_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(cut), ok, oa, m);
   KeepRule r{0, 0, 0, cut_key(cut), -1ll};
   return compact_rule<W>(c, ik, ia, n, r, ok, oa, m);
 }
@@ -428,6 +833,7 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
   if (n <= k) {
     if (tiny >= 0.0) {
       // filter only: keep |a| > tiny (all of them pass the selection)
+      if (n && n <= COOP_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(tiny), ok, oa, m);
       // tau = 0 keeping all n ties keeps everything before the tiny filter
       KeepRule r{1, 0ull, (u64)n, -1ll, cut_key(tiny)};
       return compact_rule<W>(c, ik, ia, n, r, ok, oa, m);
@@ -439,10 +845,20 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
     *m = n;
     return SFCI_OK;
   }
+  int st;
+  if (n <= COOP_MAX && k > 0) {
+    if (ok != ik) return select_coop<W>(c, ik, ia, n, 1, k, cut_key(tiny), ok, oa, m);
+    KT* tk = (KT*)scratch_get(c, "topk_k", n * sizeof(KT));
+    double* ta = (double*)scratch_get(c, "topk_a", n * sizeof(double));
+    if (!tk || !ta) return SFCI_ERR_NOMEM;
+    if ((st = select_coop<W>(c, ik, ia, n, 1, k, cut_key(tiny), tk, ta, m))) return st;
+    SFCI_CUDA(cudaMemcpyAsync(ok, tk, *m * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
+    SFCI_CUDA(cudaMemcpyAsync(oa, ta, *m * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+    return SFCI_OK;
+  }
   u64 tau;
   size_t gt;
-  int st = select_threshold(c, ia, n, k, &tau, &gt);
-  if (st) return st;
+  if ((st = select_threshold(c, ia, n, k, &tau, &gt))) return st;
   size_t need_eq = k - gt;
   if (ok == ik) {
     // compaction may not run in place across tiles; stage through scratch
@@ -500,19 +916,52 @@ __global__ void k_sumsq_part(const double* __restrict__ a, size_t n, double* __r
   if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
-__global__ void k_sum_final(const double* __restrict__ part, int np, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < np; ++i) s += __ldcg(part + i);
-    *out = s;
-  }
+// Partial sums added by one CTA.  A dependent FP64 addition takes about 150 cycles
+// on this GPU, so a serial chain over 512 partials cost 40 us (683 of a dot: 50);
+// the tree takes 3.  It adds in twice the working precision, so no rounding is
+// added to the partial sums' but the last.
+constexpr int SUM_THREADS = 256;
+
+__global__ void __launch_bounds__(SUM_THREADS) k_sum_parts(const double* __restrict__ p, u64 n, double* __restrict__ out) {
+  __shared__ double sh[2 * SUM_THREADS];
+  double hi = 0.0, lo = 0.0;
+  for (u64 i = threadIdx.x; i < n; i += SUM_THREADS) two_sum(hi, lo, __ldcg(p + i), 0.0);
+  const double t = block_sum2<SUM_THREADS>(hi, lo, sh);
+  if (threadIdx.x == 0) *out = t;
+}
+
+int sum_parts(Ctx& c, const double* p, u64 n, double* out) {
+  SFCI_LAUNCH(c, k_sum_parts, 1, SUM_THREADS, 0, p, n, out);
+  return SFCI_OK;
+}
+
+// The same with the squares (each rounded once) added in twice the working
+// precision, for vectors short enough that the seven FP64 operations an entry (an
+// SM issues two a cycle) stay below the launch and readback: 5 us at 400,000
+// entries.  The sum is then that of the squares, rounded once but for rare cases.
+constexpr size_t SUMSQ2_MAX = 1u << 20;
+constexpr int SUMSQ2_BLOCKS = 152;
+
+__global__ void __launch_bounds__(256) k_sumsq_part2(const double* __restrict__ a, size_t n, double* __restrict__ part) {
+  __shared__ double sh[512];
+  double hi = 0.0, lo = 0.0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    two_sum(hi, lo, a[i] * a[i], 0.0);
+  const double t = block_sum2<256>(hi, lo, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
 int reduce_sum_sq(Ctx& c, const double* a, size_t n, double* out) {
   double* part = (double*)scratch_get(c, "red_part", (RED_BLOCKS + 1) * sizeof(double));
   if (!part) return SFCI_ERR_NOMEM;
-  SFCI_LAUNCH(c, k_sumsq_part, RED_BLOCKS, 256, 0, a, n, part);
-  SFCI_LAUNCH(c, k_sum_final, 1, 32, 0, (const double*)part, RED_BLOCKS, part + RED_BLOCKS);
+  const int nb = n <= SUMSQ2_MAX ? SUMSQ2_BLOCKS : RED_BLOCKS;
+  if (n <= SUMSQ2_MAX) {
+    SFCI_LAUNCH(c, k_sumsq_part2, SUMSQ2_BLOCKS, 256, 0, a, n, part);
+  } else {
+    SFCI_LAUNCH(c, k_sumsq_part, RED_BLOCKS, 256, 0, a, n, part);
+  }
+  int st = sum_parts(c, part, nb, part + RED_BLOCKS);
+  if (st) return st;
   return read_words(c, part + RED_BLOCKS, sizeof(double), out);
 }
 

@@ -51,6 +51,35 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// (hi, lo) += (bh, bl), exact up to the rounding of the error terms (Knuth's two-sum)
+__device__ __forceinline__ void two_sum(double& hi, double& lo, double bh, double bl) {
+  const double s = hi + bh, t = s - hi, e = (hi - (s - t)) + (bh - t);
+  hi = s;
+  lo += bl + e;
+}
+// a compensated sum as a double (infinities and NaNs: their error terms are NaN)
+__device__ __forceinline__ double two_value(double hi, double lo) { return isfinite(hi) ? hi + lo : hi; }
+// sum of every thread's (hi, lo); valid in thread 0.  Warp 0 adds NT / 32 pairs a
+// lane before its tree: a tree over all threads would issue three times the FP64
+// additions, of which an SM takes two a cycle.
+template <int NT>
+__device__ __forceinline__ double block_sum2(double hi, double lo, double* sh /* 2 * NT */) {
+  sh[threadIdx.x] = hi;
+  sh[NT + threadIdx.x] = lo;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int q = 1; q < NT / 32; ++q) two_sum(hi, lo, sh[q * 32 + threadIdx.x], sh[NT + q * 32 + threadIdx.x]);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const double bh = __shfl_xor_sync(0xffffffffu, hi, o), bl = __shfl_xor_sync(0xffffffffu, lo, o);
+      two_sum(hi, lo, bh, bl);
+    }
+  }
+  __syncthreads();
+  return two_value(hi, lo);
+}
+
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double* sh) {
   v = warp_sum(v);
@@ -63,6 +92,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   __syncthreads();
   return r;  // valid in thread 0
 }
+
 #endif
 
 // out[i] = sum_{j<i} in[j] for i <= n (out has n+1 entries; out[n] = total).
@@ -104,8 +134,16 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
 template <int W>
 int select_sorted(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, size_t k, size_t* m);
 
+// *out = sum of the n partial sums p (device): a fixed tree in twice the working
+// precision, rounded once
+int sum_parts(Ctx& c, const double* p, u64 n, double* out);
+
 // deterministic FP64 sum / dot reductions
 int reduce_sum_sq(Ctx& c, const double* a, size_t n, double* out);
+
+// pinned host word that a kernel sets when a grid barrier ran out of its poll
+// limit; read_words and the vector download turn it into SFCI_ERR_CUDA
+unsigned* coop_error_word(Ctx& c);
 
 // device -> host readback of a few words through pinned memory (synchronises)
 int read_words(Ctx& c, const void* dptr, size_t nbytes, void* host);

@@ -133,6 +133,12 @@ struct RowArgs {
   unsigned *rsg, *rsx;   // S entries: group; i | a << 6 | phase << 12
   unsigned* rdg;         // D entries: group and element
   double* rdv;
+  // extra sources of one term each (keys and amplitudes from ns on), by row
+  u64 nx;
+  unsigned* xra;         // alpha ranks
+  uint32_t *xc, *xoff;   // per rank: count, exclusive scan
+  ST* xH;
+  double* xv;            // s * amplitude
   // units
   unsigned* bins;        // [BINS + 1] counts, then cursors at +64
   u64 unit_raw;
@@ -194,6 +200,36 @@ __global__ void k_rows_split(RowArgs<W> a) {
     a.rb[j] = rb;
     atomicAdd((unsigned*)(a.arank + ra), 1u);  // the low word: at most 2^31 sources
     a.brank[rb] = 1u;
+  }
+  if (bad) atomicOr(a.flag, 1u);
+}
+
+// extra sources: each adds one term to the row of its own alpha string (counts,
+// then entries; an extra determinant of other spin counts declines the product)
+template <int W, bool FILL>
+__global__ void k_rows_extra(RowArgs<W> a) {
+  typedef typename StrOf<W>::T ST;
+  unsigned bad = 0;
+  for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < a.nx; j += (u64)gridDim.x * blockDim.x) {
+    ST sa, sb;
+    split_key(a.keys[a.ns + j], sa, sb);
+    if (!FILL) {
+      if (spop(sa) != a.na || spop(sb) != a.nb || !key_within(a.keys[a.ns + j], a.h.N)) {
+        bad = 1;
+        a.xra[j] = ~0u;
+        continue;
+      }
+      const unsigned r = rank_of(a.bin, sa);
+      a.xra[j] = r;
+      atomicAdd(a.xc + r, 1u);
+      atomicAdd((unsigned long long*)(a.rpack + r), 1ull << RP_RAW);
+    } else {
+      const unsigned r = a.xra[j];
+      if (r == ~0u) continue;
+      const unsigned k = a.xoff[r] + atomicSub(a.xc + r, 1u) - 1u;
+      a.xH[k] = hs_of(sb);
+      a.xv[k] = signed_by(interleave_par(sa, sb), a.amps[a.ns + j]);
+    }
   }
   if (bad) atomicOr(a.flag, 1u);
 }
@@ -714,6 +750,11 @@ __global__ void __launch_bounds__(LIGHT_WARPS * 32) k_rows_light(RowArgs<W> a) {
         t.add(ok, a.pH[e], a.pc[e] * v, 0u, tb, a.max_exp, bad);
       });
     }
+    if (a.nx)
+      for (unsigned x0 = a.xoff[r], x1 = a.xoff[r + 1]; x0 < x1; x0 += 32) {
+        const unsigned x = min(x0 + lane, x1 - 1);
+        t.add(x0 + lane < x1, a.xH[x], a.xv[x], 0u, tb, a.max_exp, bad);
+      }
     __syncwarp();
     const ST rstr = unrank_warp<ST>(a.bin, r, a.na, a.h.M);
     uq += row_flush<W, DB>(a, t, rstr, 1u << tb, 0u, 32u, true);
@@ -898,6 +939,13 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
           full |= !tab.add(i0 + lane < p1 && hs_top(H) - tlo <= span, H, a.pd[p], 0u, tb, a.max_exp, bad);
         }
       }
+      // extra sources of the row (unbucketed: each step passes over them)
+      if (a.nx)
+        for (unsigned x0 = a.xoff[r] + warp * 32, x1 = a.xoff[r + 1]; x0 < x1; x0 += NT) {
+          const unsigned x = min(x0 + lane, x1 - 1);
+          const ST H = a.xH[x];
+          full |= !tab.add(x0 + lane < x1 && hs_top(H) - tlo <= span, H, a.xv[x], 0u, tb, a.max_exp, bad);
+        }
       // (3c) spin-1 doubles of the row's own sources: pieces of one source's list
       // while those are long enough for a warp, else 32 lists at a time
       if (own && a.ndb) {
@@ -977,10 +1025,13 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= n1) break;
         const unsigned te = min(n1, t + chunk);
+        // (the entry is clamped before the search: past the end it would find a
+        // group that does not hold the clamped entry)
         unsigned l = 0, h = nS;
+        const unsigned first = min(t + lane, te - 1);
         while (h - l > 1) {
           const unsigned m = (l + h) >> 1;
-          if (c_p1[m] <= t + lane) l = m; else h = m;
+          if (c_p1[m] <= first) l = m; else h = m;
         }
         // the lane's group: last entry, entry offset, first source, integral row
         unsigned pe = c_p1[l + 1], o1 = c_o1[l], gb = c_gb[l], row = c_row[l];
@@ -1106,8 +1157,8 @@ bool row_tables(Ctx& c, const HamView& h) {
 }
 
 template <int W>
-int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 ns, double lambda, double coeff,
-                 u64 cap, RowsResult<W>* out, bool* done) {
+int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 ns, u64 nx, double lambda,
+                 double coeff, u64 cap, RowsResult<W>* out, bool* done) {
   typedef typename StrOf<W>::T ST;
   typedef typename KeyOf<W>::T KT;
   *done = false;
@@ -1127,16 +1178,17 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   const u64 nsa = (u64)na * nva, nsb = (u64)nb * nvb;
   const u64 nda = (u64)(na * (na - 1) / 2) * (nva * (nva - 1) / 2), ndb = (u64)(nb * (nb - 1) / 2) * (nvb * (nvb - 1) / 2);
   const u64 conn = 1 + nsa + nsb + nda + ndb + nsa * nsb;
-  const u64 T = ns * conn;
-  if (conn >= (1ull << 16) || nsa >= (1u << RP_D) || nda >= (1u << (RP_RAW - RP_D)) || ndb >= 65536 ||
-      ns * (1 + nsb + ndb) >= (1ull << (64 - RP_RAW)) || ns * nsb >= (1ull << 31) || ns >= (1ull << 31))
+  const u64 most = conn + (nx ? 2 : 0);  // terms of one target: at most two extra vectors
+  const u64 T = ns * conn + nx;
+  if (most >= (1ull << 16) || nsa >= (1u << RP_D) || nda >= (1u << (RP_RAW - RP_D)) || ndb >= 65536 ||
+      ns * (1 + nsb + ndb) + nx >= (1ull << (64 - RP_RAW)) || nx >= (1ull << 31) || ns * nsb >= (1ull << 31) || ns >= (1ull << 31))
     return SFCI_OK;
   // Where the row form pays: its fixed part sweeps the rank tables and visits every
   // row reached, so its lead starts at more terms the more strings there are
   // (measured crossings, terms: 1.0e6 with 252 strings a spin, 1.4e7 with 1.2e6,
   // 5.3e7 with 1.8e7).
   if ((double)T < 1048576.0 + 9000.0 * std::sqrt((double)(RA + RB))) return SFCI_OK;
-  const bool d16 = conn <= (1u << 15);
+  const bool d16 = most <= (1u << 15);
   RowArgs<W> a{};
   a.h.N = c.N;
   a.h.M = M;
@@ -1161,7 +1213,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   const u64 margin = std::min<u64>(T, std::max<u64>(1ull << 24, avail / 64 / (sizeof(KT) + 8)));
   const u64 slack = (u64)c.sm_count * 10240;  // an SM's shared memory holds fewer table slots than that
   const u64 SC = std::min<u64>(cap, T) + margin + slack;
-  size_t need = RA * 40 + RB * 8 + ns * (nsb * (sizeof(ST) + 4 + 6) + 64) + SC * 2 * (sizeof(KT) + 8) + ((size_t)64 << 20);
+  size_t need = (nx ? RA * 8 + nx * (sizeof(ST) + 12) : 0) + RA * 40 + RB * 8 + ns * (nsb * (sizeof(ST) + 4 + 6) + 64) + SC * 2 * (sizeof(KT) + 8) + ((size_t)64 << 20);
   if (need > avail) return SFCI_OK;
   if (need > freeb + mine) scratch_release_plan(c);
   if (!row_tables(c, a.h)) return SFCI_OK;
@@ -1187,6 +1239,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.keys = keys;
   a.amps = amps;
   a.ns = ns;
+  a.nx = nx;
   a.lambda = lambda;
   a.coeff = coeff;
   a.RA = (unsigned)RA;
@@ -1272,11 +1325,24 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.rsx = (unsigned*)get("rw_rsx", nSent * 4);
   a.rdg = (unsigned*)get("rw_rdg", std::max<u64>(1, nDent) * 4);
   a.rdv = (double*)get("rw_rdv", std::max<u64>(1, nDent) * 8);
+  if (nx) {
+    a.xra = (unsigned*)get("rw_xra", nx * 4);
+    a.xc = (uint32_t*)get("rw_xc", RA * 4);
+    a.xoff = (uint32_t*)get("rw_xoff", (RA + 1) * 4);
+    a.xH = (ST*)get("rw_xH", nx * sizeof(ST));
+    a.xv = (double*)get("rw_xv", nx * 8);
+  }
   if (!ok) {
     phase_end(c, tok);
     return SFCI_OK;
   }
   SFCI_CUDA(cudaMemsetAsync(a.rpack, 0, RA * 8, c.stream));
+  if (nx) {
+    SFCI_CUDA(cudaMemsetAsync(a.xc, 0, RA * 4, c.stream));
+    SFCI_LAUNCH(c, (k_rows_extra<W, false>), grid_of(nx, 256), 256, 0, a);
+    if ((st = scan_excl_u32(c, a.xc, a.xoff, RA))) return st;
+    SFCI_LAUNCH(c, (k_rows_extra<W, true>), grid_of(nx, 256), 256, 0, a);
+  }
   SFCI_CUDA(cudaMemsetAsync(a.rcur, 0, RA * 8, c.stream));
   SFCI_LAUNCH(c, k_rows_groups<W>, grid_of(std::max(RA, RB), 256), 256, 0, a);
   if ((st = scan_excl(c, a.goff, a.goff, a.nG))) return st;
@@ -1308,7 +1374,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   u64 nunits = 0;
   for (int i = 0; i < BINS; ++i) nunits += bh[i];
   a.nlight = bh[BINS];
-  if (maxg >= (1u << 19) || nb0 > nb0max || nb1 > nb1max || nunits + a.nlight >= (1ull << 31)) {
+  if ((unsigned)th[1] || maxg >= (1u << 19) || nb0 > nb0max || nb1 > nb1max || nunits + a.nlight >= (1ull << 31)) {
     phase_end(c, tok);
     return SFCI_OK;
   }
@@ -1431,7 +1497,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   return SFCI_OK;
 }
 
-template int rows_product<1>(Ctx&, const u64*, const double*, u64, double, double, u64, RowsResult<1>*, bool*);
-template int rows_product<2>(Ctx&, const K128*, const double*, u64, double, double, u64, RowsResult<2>*, bool*);
+template int rows_product<1>(Ctx&, const u64*, const double*, u64, u64, double, double, u64, RowsResult<1>*, bool*);
+template int rows_product<2>(Ctx&, const K128*, const double*, u64, u64, double, double, u64, RowsResult<2>*, bool*);
 
 }  // namespace sfci

@@ -19,14 +19,15 @@ struct RowsResult {
   bool pruned = false;  // survivors were cut to the output capacity on the way
 };
 
-// The product's terms generated and merged row by row (see rows.cu).  *done is
+// The product's terms generated and merged row by row (see rows.cu), with nx extra
+// sources after the ns determinants of one term each (key, amplitude).  *done is
 // false when the input is outside what the row form handles (the caller then
 // runs the partitioned pipeline): mixed spin counts, more rows or pairs than
 // its tables take, too little device memory, or a term too large for its
 // accumulators.
 template <int W>
-int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 ns, double lambda, double coeff,
-                 u64 cap, RowsResult<W>* out, bool* done);
+int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 ns, u64 nx, double lambda,
+                 double coeff, u64 cap, RowsResult<W>* out, bool* done);
 
 // device memory of the row form's per-context tables
 void rows_free(Ctx& c);

@@ -1256,14 +1256,6 @@ __global__ void k_table_build(const KT* __restrict__ keys, const double* __restr
   }
 }
 
-__global__ void k_sum_parts(const double* __restrict__ p, int n, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += __ldcg(p + i);
-    *out = s;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------
@@ -1579,15 +1571,15 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
       return set_error(SFCI_ERR_UNSUPPORTED, "SpMSpV: determinants connect to more than 2^19 others");
   }
   // Row-driven form: whole products on one plain Hamiltonian.  The partitioned
-  // pipeline below takes the rest (extra sources, screens, batches), the plans a
+  // pipeline below takes the rest (sums of squares, screens, batches), the plans a
   // caller asked for by a device budget or by class passes, and what
   // rows_product declines.
-  if (ng == ns && !c.screen && !c.ninst && !c.opts.mem_budget && c.tune_class_passes <= 0 &&
+  if (!(ex && ex->sumsq) && !(c.screen && ng == ns) && !c.ninst && !c.opts.mem_budget && c.tune_class_passes <= 0 &&
       ns * conn >= ROWS_MIN_TERMS) {
     RowsResult<W> rr;
     bool done = false;
     phase_end(c, tok);
-    if ((st = rows_product<W>(c, src_k, src_a, ns, lambda, coeff, out.cap, &rr, &done))) return st;
+    if ((st = rows_product<W>(c, gen_k, gen_a, ns, ng - ns, lambda, coeff, out.cap, &rr, &done))) return st;
     if (done) {
       c.stats[1] = rr.terms;
       c.stats[2] = rr.uniq;
@@ -2105,7 +2097,7 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
     for (int i = 0; i < INST_MAX; ++i) c.inst_diag[i] = fx_to_double(dx[2 + 2 * i], dx[3 + 2 * i]);
   }
   if (qpart) {
-    SFCI_LAUNCH(c, k_sum_parts, 1, 32, 0, (const double*)qpart, (int)leafgrid, qpart + leafgrid);
+    if ((st = sum_parts(c, qpart, leafgrid, qpart + leafgrid))) return st;
     double q2[2] = {0.0, 0.0};
     if ((st = read_words(c, qpart + leafgrid, 2 * sizeof(double), q2))) return st;
     *ex->sumsq = q2[0] + q2[1];
@@ -2165,7 +2157,7 @@ int energy_impl(Ctx& c, const Vec& psi, double* E) {
   g.tmask = (unsigned)(tsz - 1);
   g.epart = part;
   if ((st = launch_gen<W, M_ENERGY>(c, g, G, 0))) return st;
-  SFCI_LAUNCH(c, k_sum_parts, 1, 32, 0, (const double*)part, (int)G, part + G);
+  if ((st = sum_parts(c, part, G, part + G))) return st;
   return read_words(c, part + G, sizeof(double), E);
 }
 
@@ -2209,14 +2201,6 @@ __global__ void __launch_bounds__(256) k_proj_dot(const KT* __restrict__ keys, c
   }
   acc = block_sum<256>(acc, s_red);
   if (threadIdx.x == 0) part[blockIdx.x] = acc;
-}
-
-__global__ void k_proj_sum(const double* __restrict__ part, int G, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < G; ++b) s += __ldcg(part + b);
-    *out = s;
-  }
 }
 
 // out[j] = <basis_j | merge((H - lambda) src)> for j < nv (src coefficient 1):
@@ -2297,7 +2281,7 @@ int project_impl(Ctx& c, const Vec& src, double lambda, const Vec* const* basis,
     const unsigned dg = (unsigned)std::min<u64>((l + 255) / 256, DG);
     SFCI_LAUNCH(c, k_proj_dot<KT>, dg, 256, 0, (const KT*)basis[j]->keys, (const double*)basis[j]->amps, l,
                 (const KT*)tk, (unsigned)(tsz - 1), (const u64*)plo, (const u64*)phi, pj);
-    SFCI_LAUNCH(c, k_proj_sum, 1, 32, 0, (const double*)pj, (int)dg, pj + DG);
+    if ((st = sum_parts(c, pj, dg, pj + DG))) return st;
   }
   std::vector<double> all((u64)nv * (DG + 1));
   if ((st = read_words(c, part, all.size() * sizeof(double), all.data()))) return st;

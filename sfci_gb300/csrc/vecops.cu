@@ -57,14 +57,15 @@ __global__ void k_merge(const KT* __restrict__ A, const double* __restrict__ Aa,
   }
 }
 
-// dot over common keys (keys unique within each vector)
+// dot over common keys (keys unique within each vector); the products of matches,
+// a few a thread, are summed in twice the working precision
 template <class KT>
 __global__ void k_dot(const KT* __restrict__ A, const double* __restrict__ Aa, u64 na, const KT* __restrict__ B,
                       const double* __restrict__ Ba, u64 nb, double* __restrict__ part) {
-  __shared__ double sh[32];
+  __shared__ double sh[2 * MP_THREADS];
   const u64 n = na + nb;
   u64 d = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * MP_ITEMS;
-  double acc = 0.0;
+  double acc = 0.0, low = 0.0;
   if (d < n) {
     u64 i = merge_path(A, na, B, nb, d), j = d - i;
     for (int t = 0; t < MP_ITEMS && d + t < n; ++t) {
@@ -72,21 +73,13 @@ __global__ void k_dot(const KT* __restrict__ A, const double* __restrict__ Aa, u
       if (takeA) {
         ++i;
       } else {
-        if (i > 0 && key_eq(A[i - 1], B[j])) acc += Aa[i - 1] * Ba[j];
+        if (i > 0 && key_eq(A[i - 1], B[j])) two_sum(acc, low, Aa[i - 1] * Ba[j], 0.0);
         ++j;
       }
     }
   }
-  double t = block_sum<MP_THREADS>(acc, sh);
+  const double t = block_sum2<MP_THREADS>(acc, low, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
-__global__ void k_sum_serial(const double* __restrict__ p, u64 n, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (u64 i = 0; i < n; ++i) s += __ldcg(p + i);
-    *out = s;
-  }
 }
 
 // ---- segmented reduction of runs of equal keys (sorted input) -------------
@@ -185,7 +178,8 @@ int dot_impl(Ctx& c, const Vec& x, const Vec& y, double* out) {
   if (!part) return SFCI_ERR_NOMEM;
   SFCI_LAUNCH(c, k_dot<KT>, (unsigned)grid, MP_THREADS, 0, (const KT*)x.keys, x.amps, x.len, (const KT*)y.keys,
               y.amps, y.len, part);
-  SFCI_LAUNCH(c, k_sum_serial, 1, 32, 0, (const double*)part, grid, part + grid);
+  int st = sum_parts(c, part, grid, part + grid);
+  if (st) return st;
   return read_words(c, part + grid, sizeof(double), out);
 }
 

@@ -90,3 +90,30 @@ def test_inputs_the_row_form_declines(tmp_path):
         if not fails:
             assert np.array_equal(got[0][0], got[1][0]) and got[0][2] == got[1][2]
             assert np.array_equal(got[0][1].view(np.uint64), got[1][1].view(np.uint64))
+
+
+@pytest.mark.parametrize("M,na,nb,n", [(14, 5, 5, 2500), (28, 5, 6, 1200), (34, 5, 5, 1601)])
+def test_extra_sources_join_their_rows(M, na, nb, n, tmp_path):
+    """The linear solver's product (two vectors removed before the cut): extra terms
+    on determinants the product reaches, and on some far from every source, whose
+    rows hold nothing else."""
+    path = str(tmp_path / "sys_IN")
+    fd.rhf_to_in_file(path, M, na + nb, 3)
+    rng = np.random.default_rng(13)
+    keys, amps = vector(M, na, nb, n, rng)
+    far = sorted({sum(1 << 2 * int(i) for i in M - 1 - np.arange(na)) |
+                  sum(2 << 2 * int(i) for i in M - 1 - rng.choice(M // 2, nb, replace=False)) for _ in range(40)})
+    far = sg.keys_from_ints(far, 1 if M <= 32 else 2)
+    basis = [(np.concatenate([keys[1::3], far]), rng.standard_normal(len(keys[1::3]) + len(far))),
+             (keys[::2], rng.standard_normal(len(keys[::2]))), (keys, amps)]
+    got = []
+    for budget in (0, 64 << 30):
+        c = sg.Context(path, 2 * M, na + nb, Nd=n, coeff_cut=1e-7, mem_budget=budget)
+        vecs = [c.vec_from(k, a) for k, a in basis]
+        out = c.vec(2000000)
+        for pair in (vecs, vecs[::2]):
+            h = c.spmspvm_bucket_linear(vecs[2], out, 0.75, pair)
+            got.append((*out.download(), h, c.last_stats()["terms"]))
+    for x, y in zip(got[:2], got[2:]):
+        assert np.array_equal(x[0], y[0]) and np.array_equal(x[1].view(np.uint64), y[1].view(np.uint64))
+        assert np.array_equal(x[2], y[2]) and x[3] == y[3]
