@@ -68,6 +68,11 @@ constexpr int MID_THREADS = 128, MID_TB = 10;
 template <int W> struct Big { static constexpr int threads = 512, tb = 12; };
 template <> struct Big<2> { static constexpr int threads = 256, tb = 11; };
 constexpr float LOAD = 0.65f;               // share of a table's slots a step aims to fill
+// terms per distinct target the first step of a unit assumes (later steps follow
+// the density seen).  With the previous product's mean (3.2 at 120,000 sources) a
+// tenth of the steps overflowed and were redone; with 2, one in two thousand (a
+// row has no more distinct targets than there are beta strings, either)
+constexpr float FIRST_DUP = 2.0f;
 constexpr int MID_BIN = 12;                // MID_MAX = 2^MID_BIN - 1 terms
 constexpr unsigned D1_PIECE = 128;         // entries of one source's doubles a warp takes at a time
 constexpr unsigned PROBE_MAX = 64;         // probes before a table counts as full
@@ -148,7 +153,6 @@ struct RowArgs {
   unsigned* ucur;        // work counters
   uint4* redo;
   unsigned* nredo;
-  float dup;             // expected terms per distinct target
   // survivors
   FxCut cut;
   KT* sk;
@@ -541,13 +545,8 @@ struct RowTable {
   unsigned* w;
   unsigned n;  // word stride
 
-  // Add (flip ? -x : x) to H's sum, for the lanes with `act`; every lane of the
-  // warp calls it, so that the lanes that claimed a slot and those that found
-  // theirs go on together (left to itself the compiler ran the two groups one
-  // after the other through the rounding and the reductions).  False: no free slot.
-  __device__ __forceinline__ bool add(bool act, ST H, double x, unsigned flip, int tb, int max_exp,
-                                      unsigned& bad) const {
-    const int s = slot<true>(act, H, tb);
+  // Add (flip ? -x : x) to the sum of slot s (-1: nothing).
+  __device__ __forceinline__ void acc(int s, double x, unsigned flip, int max_exp, unsigned& bad) const {
     // x on the FX_FRAC grid, nearest, ties to even, as in fx_addends
     const u64 b = dbl_bits(x);
     const int e = (int)((b >> 52) & 0x7ff);
@@ -578,7 +577,32 @@ struct RowTable {
         if (t) atomicAdd(p + 4 * n, (t ^ neg) - neg);
       }
     }
+  }
+  // Add to H's sum, for the lanes with `act`; every lane of the warp calls it, so
+  // that the lanes that claimed a slot and those that found theirs go on together
+  // (left to itself the compiler ran the two groups one after the other through the
+  // rounding and the reductions).  False: no free slot.
+  __device__ __forceinline__ bool add(bool act, ST H, double x, unsigned flip, int tb, int max_exp,
+                                      unsigned& bad) const {
+    const int s = slot<true>(act, H, tb);
+    acc(s, x, flip, max_exp, bad);
     return !act || s >= 0;
+  }
+  // two entries a lane: their bucket loads overlap and share the probe loop
+  __device__ __forceinline__ bool add2(bool a0, ST H0, double x0, unsigned f0, bool a1, ST H1, double x1, unsigned f1,
+                                       int tb, int max_exp, unsigned& bad) const {
+    const unsigned mask = (1u << (tb - 2)) - 1u;
+    unsigned b0 = hs_slot(H0, tb - 2), b1 = hs_slot(H1, tb - 2);
+    int s0 = -1, s1 = -1;
+    bool p0 = a0, p1 = a1;
+    for (unsigned probe = 0; probe < PROBE_MAX; ++probe) {
+      look<true>(p0, H0, b0, s0, mask);
+      look<true>(p1, H1, b1, s1, mask);
+      if (!__any_sync(0xffffffffu, p0 || p1)) break;
+    }
+    acc(s0, x0, f0, max_exp, bad);
+    acc(s1, x1, f1, max_exp, bad);
+    return (!a0 || s0 >= 0) && (!a1 || s1 >= 0);
   }
   static __device__ __forceinline__ uint32_t cas(uint32_t* p, uint32_t v) { return atomicCAS(p, 0u, v); }
   static __device__ __forceinline__ u64 cas(u64* p, u64 v) {
@@ -601,45 +625,50 @@ struct RowTable {
     }
   }
   // Slot of H for the lanes with `act`, claimed when CLAIM; -1: not there (or no
-  // free slot within the probe limit).  Slots form buckets of 16 bytes, read with
-  // one load and filled in order, so a warp rarely needs a second probe: with
+  // free slot within the probe limit).  Slots form buckets of four, read with one
+  // or two 16-byte loads and filled in order, so a warp rarely needs a second probe: with
   // single-slot probing the slowest of 32 lanes took five or six at the same load.
   template <bool CLAIM>
   __device__ __forceinline__ int slot(bool act, ST H, int tb) const {
-    constexpr int BS = 16 / sizeof(ST), BB = sizeof(ST) == 4 ? 2 : 1;
-    const unsigned mask = (1u << (tb - BB)) - 1u;
-    unsigned b = hs_slot(H, tb - BB);
+    const unsigned mask = (1u << (tb - 2)) - 1u;
+    unsigned b = hs_slot(H, tb - 2);
     int s = -1;
     for (unsigned probe = 0; probe < PROBE_MAX; ++probe) {
-      if (act) {
-        ST v[BS];
-        load_bucket(k + b * BS, v);
-        int hit = -1, free = -1;
-#pragma unroll
-        for (int i = BS - 1; i >= 0; --i) {
-          if (v[i] == H) hit = i;
-          if (v[i] == 0) free = i;
-        }
-        if (hit >= 0) {
-          s = (int)(b * BS) + hit;
-          act = false;
-        } else if (free >= 0) {
-          if (CLAIM) {  // (when another key took it, the bucket is looked at again)
-            const ST old = cas(k + b * BS + free, H);
-            if (old == 0 || old == H) {
-              s = (int)(b * BS) + free;
-              act = false;
-            }
-          } else {
-            act = false;
-          }
-        } else {
-          b = (b + 1) & mask;
-        }
-      }
+      look<CLAIM>(act, H, b, s, mask);
       if (!__any_sync(0xffffffffu, act)) break;
     }
     return s;
+  }
+  // one probe: clears `act` when H was found (s), claimed (s) or, unless CLAIM, is absent
+  template <bool CLAIM>
+  __device__ __forceinline__ void look(bool& act, ST H, unsigned& b, int& s, unsigned mask) const {
+    constexpr int BS = 4;
+    if (act) {
+      ST v[BS];
+      load_bucket(k + b * BS, v);
+      int hit = -1, free = -1;
+#pragma unroll
+      for (int i = BS - 1; i >= 0; --i) {
+        if (v[i] == H) hit = i;
+        if (v[i] == 0) free = i;
+      }
+      if (hit >= 0) {
+        s = (int)(b * BS) + hit;
+        act = false;
+      } else if (free >= 0) {
+        if (CLAIM) {  // (when another key took it, the bucket is looked at again)
+          const ST old = cas(k + b * BS + free, H);
+          if (old == 0 || old == H) {
+            s = (int)(b * BS) + free;
+            act = false;
+          }
+        } else {
+          act = false;
+        }
+      } else {
+        b = (b + 1) & mask;
+      }
+    }
   }
   static __device__ __forceinline__ void load_bucket(const uint32_t* p, uint32_t* v) {
     asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -647,9 +676,9 @@ struct RowTable {
                  : "r"((unsigned)__cvta_generic_to_shared(p)));
   }
   static __device__ __forceinline__ void load_bucket(const u64* p, u64* v) {
-    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];"
-                 : "=l"(v[0]), "=l"(v[1])
-                 : "r"((unsigned)__cvta_generic_to_shared(p)));
+    const unsigned q = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "r"(q));
+    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2 + 16];" : "=l"(v[2]), "=l"(v[3]) : "r"(q));
   }
 };
 
@@ -837,7 +866,8 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
     }
     // step width: distinct targets are at most the terms of the step
     const float target = LOAD * CTA_SLOTS;
-    u64 width = (u64)fminf(4294967296.0f, fmaxf(1.0f, 4294967296.0f * target * a.dup / raw));
+    const float guess = fminf(raw * (1.0f / FIRST_DUP), (float)a.RB);  // distinct targets of the row
+    u64 width = (u64)fminf(4294967296.0f, fmaxf(1.0f, 4294967296.0f * target / guess));
     bool wide = false;  // a table sized for this row's mean density was too small
     u64 lo = un.y;
     const u64 end = (u64)un.z + 1;
@@ -1018,7 +1048,7 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
       // which warps take a chunk at a time (lane 0 decides for the warp: the
       // loops hold warp collectives); each lane follows the group its entry is in
       const unsigned n1 = c_p1[nS];
-      const unsigned chunk = min(256u, max(32u, (n1 / (NWARP * 8)) & ~31u));
+      const unsigned chunk = min(256u, max(64u, (n1 / (NWARP * 8)) & ~63u));
       for (;;) {
         unsigned t = 0;
         if (lane == 0) t = *(volatile unsigned*)&s_ovf ? ~0u : atomicAdd(&s_w1, chunk);
@@ -1035,8 +1065,7 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
         }
         // the lane's group: last entry, entry offset, first source, integral row
         unsigned pe = c_p1[l + 1], o1 = c_o1[l], gb = c_gb[l], row = c_row[l];
-        for (; t < te; t += 32) {
-          const unsigned i = min(t + lane, te - 1);
+        auto entry = [&](unsigned i, ST& H, double& v, unsigned& par) {
           if (i >= pe) {
             do ++l; while (c_p1[l + 1] <= i);
             pe = c_p1[l + 1];
@@ -1045,11 +1074,19 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
             row = c_row[l];
           }
           const unsigned e = o1 + i;
-          const ST H = a.eH[e];
+          H = a.eH[e];
           const uint32_t y = a.ex[e];
-          const bool act = t + lane < te && hs_top(H) - tlo <= span;
-          const double v = a.pc[gb + (y >> 13)] * SFCI_LDG(a.os + (row & 0x7fffffffu) + (y & 0xfffu));
-          full |= !tab.add(act, H, v, (row >> 31) ^ ((y >> 12) & 1u), tb, a.max_exp, bad);
+          v = a.pc[gb + (y >> 13)] * SFCI_LDG(a.os + (row & 0x7fffffffu) + (y & 0xfffu));
+          par = (row >> 31) ^ ((y >> 12) & 1u);
+        };
+        for (; t < te; t += 64) {
+          ST H0, H1;
+          double v0, v1;
+          unsigned f0, f1;
+          entry(min(t + lane, te - 1), H0, v0, f0);
+          entry(min(t + 32 + lane, te - 1), H1, v1, f1);
+          const bool a0 = t + lane < te && hs_top(H0) - tlo <= span, a1 = t + 32 + lane < te && hs_top(H1) - tlo <= span;
+          full |= !tab.add2(a0, H0, v0, f0, a1, H1, v1, f1, tb, a.max_exp, bad);
         }
         if (full) s_ovf = 1;
       }
@@ -1396,7 +1433,6 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.cut = fx_cut(c.opts.coeff_cut);
   a.smax = (unsigned)nsa;
   a.max_exp = d16 ? 15 : 10;
-  a.dup = c.dup_est > 1.0 ? (float)c.dup_est : 2.0f;
   SFCI_CUDA(cudaMemsetAsync(scount, 0, 4 * 8, c.stream));
   SFCI_CUDA(cudaMemsetAsync(a.c0, 0, (nb0 + 1) * 4, c.stream));
   SFCI_CUDA(cudaMemsetAsync(a.c1, 0, (nb1 + 1) * 4, c.stream));
