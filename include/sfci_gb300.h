@@ -308,6 +308,9 @@ int sfci_screen_stats(const sfci_screen* s, uint64_t* sources, uint64_t* example
  * prob_cap entries) receives each group's probability, source by source. */
 int sfci_screen_predict(sfci_screen* s, const sfci_vec* in, double threshold, uint64_t* groups,
                         uint64_t* kept_groups, uint64_t* kept_terms, float* prob_host, uint64_t prob_cap);
+/* The number of groups of the determinants of `in` (what prob_cap of
+ * sfci_screen_predict has to hold), without running the network. */
+int sfci_screen_groups(sfci_screen* s, const sfci_vec* in, uint64_t* groups);
 /* FP32 parameters (sfci_screen_param_count floats: W1[576][256] by input row,
  * b1, W2[256 out][256 in], b2, w3, b3, padding); get and/or set (nullable). */
 uint64_t sfci_screen_param_count(void);

@@ -110,6 +110,7 @@ def _sigs(L):
     L.sfci_screen_train.argtypes = [_vp, C.c_int, C.c_int, C.c_double, C.c_double, C.c_int, C.POINTER(C.c_double)]
     L.sfci_screen_stats.argtypes = [_vp, _u64p, _u64p, _u64p, _u64p]
     L.sfci_screen_predict.argtypes = [_vp, _vp, C.c_double, _u64p, _u64p, _u64p, _vp, C.c_uint64]
+    L.sfci_screen_groups.argtypes = [_vp, _vp, _u64p]
     L.sfci_screen_param_count.restype = C.c_uint64
     L.sfci_screen_params.argtypes = [_vp, _vp, _vp, C.c_uint64]
     L.sfci_screen_grads.argtypes = [_vp, _vp, C.c_uint64]
@@ -542,8 +543,9 @@ class Screen:
         return out
 
     def groups_of(self, vin: "SpVec") -> int:
-        g, kg, kt = C.c_uint64(), C.c_uint64(), C.c_uint64()
-        _check(self.L.sfci_screen_predict(self.h, vin.h, 0.5, C.byref(g), C.byref(kg), C.byref(kt), None, 0))
+        # (counting needs no inference: predict(probs=True) ran the network twice, once for this)
+        g = C.c_uint64()
+        _check(self.L.sfci_screen_groups(self.h, vin.h, C.byref(g)))
         return g.value
 
     def params(self) -> np.ndarray:

@@ -1814,6 +1814,22 @@ extern "C" int sfci_screen_predict(sfci_screen* x, const sfci_vec* in, double th
   return SFCI_OK;
 }
 
+extern "C" int sfci_screen_groups(sfci_screen* x, const sfci_vec* in, uint64_t* groups) {
+  if (!x || !in || !groups) return set_error(SFCI_ERR_ARG, "sfci_screen_groups: null argument");
+  if (!x->s.ctx || in->v.ctx != x->s.ctx)
+    return set_error(SFCI_ERR_ARG, "sfci_screen_groups: a vector of the screen's own (live) context");
+  Ctx& c = *x->s.ctx;
+  int st;
+  u64* go = (u64*)scratch_get(c, "sc_goff", (in->v.len + 1) * sizeof(u64));
+  if (!go) return SFCI_ERR_NOMEM;
+  if ((st = c.W == 1 ? group_offsets<1>(c, in->v.keys, in->v.len, go) : group_offsets<2>(c, in->v.keys, in->v.len, go)))
+    return st;
+  u64 ng = 0;
+  if ((st = read_words(c, go + in->v.len, sizeof(u64), &ng))) return st;
+  *groups = ng;
+  return SFCI_OK;
+}
+
 extern "C" int sfci_screen_params(sfci_screen* x, float* get, const float* set, uint64_t n) {
   if (!x) return set_error(SFCI_ERR_ARG, "sfci_screen_params: null screen");
   if (n != NPARAM) return set_error(SFCI_ERR_ARG, "sfci_screen_params: n must be the parameter count");

@@ -666,7 +666,7 @@ struct RowTable {
           act = false;
         }
       } else {
-        b = (b + 1) & mask;
+        b = (b + 1u + (unsigned)(H & 6u)) & mask;  // (odd: every bucket is reached)
       }
     }
   }
