@@ -494,6 +494,9 @@ int sfci_ctx_destroy(sfci_ctx* x) {
     cudaEventDestroy(p.second.first);
     cudaEventDestroy(p.second.second);
   }
+  if (c.ev_fork) cudaEventDestroy(c.ev_fork);
+  if (c.ev_join) cudaEventDestroy(c.ev_join);
+  if (c.side) cudaStreamDestroy(c.side);
   if (c.h_coop) cudaFreeHost(c.h_coop);
   if (c.h_pin) cudaFreeHost(c.h_pin);
   if (c.stream) cudaStreamDestroy(c.stream);

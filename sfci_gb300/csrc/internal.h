@@ -47,6 +47,9 @@ struct Ctx {
   // row-driven products (rows.cu): oriented opposite-spin integrals, binomials
   double* d_row_os = nullptr;  // and the directed integrals of the singles after them
   unsigned* d_row_bin = nullptr;
+  // second stream of the row-driven products (forked from and joined to `stream` by events)
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t stream = nullptr;
   int sm_count = 0;
   std::map<std::string, Buf> scratch;

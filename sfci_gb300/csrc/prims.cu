@@ -163,9 +163,11 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const KT* __restrict_
 // by the latency of its phases (about 17 us a pass at 500,000 entries, of which
 // the barriers take 4).  Measured for 56-bit keys, us, launches -> one kernel: 860
 // entries 162 -> 30, 50,000 213 -> 67, 500,000 288 -> 119, 2,000,000 533 -> 254,
-// 4,000,000 945 -> 655; 68-bit keys 500,000 391 -> 177.  Digits of 8, 9 and 10 bits
+// 4,000,000 945 -> 655, 6,000,000 1400 -> 1290 (12,000,000: 2490 -> 3660, so longer
+// ones keep the launches); 68-bit keys 500,000 391 -> 177.  Digits of 8, 9 and 10 bits
 // are within 10% of one another.
-constexpr size_t COOP_MAX = 1u << 22;
+constexpr size_t COOP_MAX = 6u << 20;      // sort
+constexpr size_t SEL_MAX = 1ull << 31;     // selection: faster at every size (30,000,000 entries 0.44 against 0.97 ms)
 constexpr int CO_THREADS = 1024;
 constexpr int CO_WARPS = CO_THREADS / 32;
 constexpr int CO_DIGIT = 8;
@@ -609,7 +611,7 @@ static int compact_rule(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia
   return SFCI_OK;
 }
 
-// ---- selection and compaction in one launch (up to COOP_MAX entries) ---------------
+// ---- selection and compaction in one launch ------------------------------------------
 // The launches above read a histogram back after each of six digits and the
 // counts after that: eight round trips to the host.  Here the digits, the counts
 // and the compaction are one cooperative kernel with a grid barrier in place of
@@ -619,7 +621,7 @@ static int compact_rule(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia
 struct SelArgs {
   const double* a;
   unsigned n, slice;
-  int mode;            // 0: keep |a| above lb only; 1: the k largest first
+  int mode;            // 0: keep |a| above lb only; 1: the k largest first; 2: with every tie of the k-th
   u64 k;
   long long low_key;   // keep bits above this as well (-1: everything)
   uint32_t* hist;      // [6][4096], zero
@@ -642,7 +644,7 @@ __global__ void __launch_bounds__(CO_THREADS, 1) k_sel_coop(SelArgs s, const KT*
   const unsigned w0 = min(s.n, b * s.slice + warp * ws), w1 = min(s.n, w0 + ws);
   unsigned target = 0;
   u64 lb = 0, tau = ~0ull, need_eq = 0;  // keep bits >= lb, and need_eq of those equal to tau
-  if (s.mode == 1) {
+  if (s.mode) {
     const int shifts[6] = {51, 39, 27, 15, 3, 0}, widths[6] = {12, 12, 12, 12, 12, 3};
     u64 prefix = 0, need = s.k;
     bool whole = false;
@@ -695,7 +697,7 @@ __global__ void __launch_bounds__(CO_THREADS, 1) k_sel_coop(SelArgs s, const KT*
     if (!whole) {
       tau = prefix;
       lb = tau + 1;
-      need_eq = need;
+      need_eq = s.mode == 2 ? ~0ull : need;
     }
   }
   const u64 low = (u64)(s.low_key + 1);
@@ -775,7 +777,8 @@ __global__ void __launch_bounds__(CO_THREADS, 1) k_sel_coop(SelArgs s, const KT*
   }
 }
 
-// mode 0: entries with bits above low_key; mode 1: the k largest first (0 < k < n)
+// mode 0: entries with bits above low_key; 1: the k largest first; 2: the same with
+// every entry tied with the k-th (0 < k < n)
 template <int W>
 static int select_coop(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, int mode, size_t k,
                        long long low_key, typename KeyOf<W>::T* ok, double* oa, size_t* m) {
@@ -797,8 +800,8 @@ static int select_coop(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia,
   s.cnt = buf + 4 + 6 * 4096;
   s.err = err;
   const unsigned G = (unsigned)((n + s.slice - 1) / s.slice);
-  SFCI_CUDA(cudaMemsetAsync(buf, 0, (mode == 1 ? 4 + 6 * 4096 : 4) * sizeof(uint32_t), c.stream));
-  const size_t sm = mode == 1 ? SEL_COPIES * 4096 * sizeof(uint32_t) : 0;
+  SFCI_CUDA(cudaMemsetAsync(buf, 0, (mode ? 4 + 6 * 4096 : 4) * sizeof(uint32_t), c.stream));
+  const size_t sm = mode ? SEL_COPIES * 4096 * sizeof(uint32_t) : 0;
   SFCI_CUDA(cudaFuncSetAttribute(k_sel_coop<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(SEL_COPIES * 4096 * sizeof(uint32_t))));
   void* args[] = {&s, &ik, &ok, &oa};
@@ -821,7 +824,7 @@ int compact_top(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t
 template <int W>
 int compact_cut(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, double cut,
                 typename KeyOf<W>::T* ok, double* oa, size_t* m) {
-  if (n && n <= COOP_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(cut), ok, oa, m);
+  if (n && n <= SEL_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(cut), ok, oa, m);
   KeepRule r{0, 0, 0, cut_key(cut), -1ll};
   return compact_rule<W>(c, ik, ia, n, r, ok, oa, m);
 }
@@ -833,7 +836,7 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
   if (n <= k) {
     if (tiny >= 0.0) {
       // filter only: keep |a| > tiny (all of them pass the selection)
-      if (n && n <= COOP_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(tiny), ok, oa, m);
+      if (n && n <= SEL_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(tiny), ok, oa, m);
       // tau = 0 keeping all n ties keeps everything before the tiny filter
       KeepRule r{1, 0ull, (u64)n, -1ll, cut_key(tiny)};
       return compact_rule<W>(c, ik, ia, n, r, ok, oa, m);
@@ -846,7 +849,7 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
     return SFCI_OK;
   }
   int st;
-  if (n <= COOP_MAX && k > 0) {
+  if (n <= SEL_MAX && k > 0) {
     if (ok != ik) return select_coop<W>(c, ik, ia, n, 1, k, cut_key(tiny), ok, oa, m);
     KT* tk = (KT*)scratch_get(c, "topk_k", n * sizeof(KT));
     double* ta = (double*)scratch_get(c, "topk_a", n * sizeof(double));
@@ -876,8 +879,22 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
 template <int W>
 int select_sorted(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, size_t k, size_t* m) {
   typedef typename KeyOf<W>::T KT;
-  int st = radix_sort_pairs<W>(c, keys, vals, n, c.N);
-  if (st) return st;
+  int st;
+  if (n > k) {
+    KT* tk = (KT*)scratch_get(c, "rs_keys", n * sizeof(KT));
+    double* ta = (double*)scratch_get(c, "rs_vals", n * sizeof(double));
+    if (!tk || !ta) return SFCI_ERR_NOMEM;
+    if (k > 0 && n <= SEL_MAX) {
+      // by magnitude first, so that only what is kept is sorted; ties of the k-th
+      // all stay until the keys are in order
+      size_t kept = 0;
+      if ((st = select_coop<W>(c, keys, vals, n, 2, k, -1ll, tk, ta, &kept))) return st;
+      SFCI_CUDA(cudaMemcpyAsync(keys, tk, kept * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
+      SFCI_CUDA(cudaMemcpyAsync(vals, ta, kept * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+      n = kept;
+    }
+  }
+  if ((st = radix_sort_pairs<W>(c, keys, vals, n, c.N))) return st;
   if (n <= k) {
     *m = n;
     return SFCI_OK;

@@ -1193,6 +1193,35 @@ bool row_tables(Ctx& c, const HamView& h) {
   return true;
 }
 
+// Work on the context's second stream: begin() orders it after what the main
+// stream holds, end() marks its end, and the main stream waits for it at join() or
+// when the object goes out of scope, whichever way the product returns.
+struct SideWork {
+  Ctx& c;
+  bool open = false;
+  explicit SideWork(Ctx& c_) : c(c_) {}
+  ~SideWork() { join(); }
+  int begin() {
+    if (!c.side) {
+      SFCI_CUDA(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
+      SFCI_CUDA(cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
+      SFCI_CUDA(cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
+    }
+    SFCI_CUDA(cudaEventRecord(c.ev_fork, c.stream));
+    SFCI_CUDA(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+    return SFCI_OK;
+  }
+  int end() {
+    open = true;
+    SFCI_CUDA(cudaEventRecord(c.ev_join, c.side));
+    return SFCI_OK;
+  }
+  void join() {
+    if (open) cudaStreamWaitEvent(c.stream, c.ev_join, 0);
+    open = false;
+  }
+};
+
 template <int W>
 int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 ns, u64 nx, double lambda,
                  double coeff, u64 cap, RowsResult<W>* out, bool* done) {
@@ -1382,6 +1411,15 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   }
   SFCI_CUDA(cudaMemsetAsync(a.rcur, 0, RA * 8, c.stream));
   SFCI_LAUNCH(c, k_rows_groups<W>, grid_of(std::max(RA, RB), 256), 256, 0, a);
+  // the beta strings' doubles need nothing but the strings: beside the lists below
+  SideWork side(c);
+  if (ndb) {
+    if ((st = side.begin())) return st;
+    k_rows_bdoubles<W><<<grid_of(a.nB, 1), 256, sizeof(uint32_t) << db, c.side>>>(a);
+    c.launches++;
+    SFCI_CUDA(cudaGetLastError());
+    if ((st = side.end())) return st;
+  }
   if ((st = scan_excl(c, a.goff, a.goff, a.nG))) return st;
   // slices per group so that a few thousand warps share the moves
   const unsigned nslice = (unsigned)std::max<u64>(1, std::min<u64>((nda + 31) / 32, 8192 / std::max(1u, a.nG)));
@@ -1446,7 +1484,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   SFCI_LAUNCH(c, (k_rows_list1<W, true>), grid_of(ns, 8), 256, 0, a);
   SFCI_LAUNCH(c, (k_rows_alpha<W, true>), ag, 256, 0, a, nslice);
   SFCI_LAUNCH(c, (k_rows_units<W, true>), grid_of(RA, 2048), 256, 0, a);
-  if (ndb) SFCI_LAUNCH(c, k_rows_bdoubles<W>, grid_of(a.nB, 1), 256, sizeof(uint32_t) << db, a);
+  side.join();
   phase_end(c, tok);
   // the rows
   tok = phase_begin(c, PH_MERGE);
@@ -1473,6 +1511,14 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   u64 nsurv = 0;
   out->units = nall;
   for (;;) {
+    // Large rows first; the smaller ones on the second stream, so that their CTAs
+    // take the SMs that the last large rows leave.
+    const bool both = nbig && (nunits > nbig || a.nlight);
+    cudaStream_t small = c.stream;
+    if (both) {
+      if ((st = side.begin())) return st;
+      small = c.side;
+    }
     if (nbig) {
       RowArgs<W> q = a;
       q.nunits = (unsigned)nbig;
@@ -1483,10 +1529,19 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
       q.units = a.units + nbig;
       q.nunits = (unsigned)(nunits - nbig);
       q.ucur = a.ucur + 1;
-      SFCI_LAUNCH(c, km, std::min(q.nunits, gm), MID_THREADS, smm, q);
+      km<<<std::min(q.nunits, gm), MID_THREADS, smm, small>>>(q);
+      c.launches++;
+      SFCI_CUDA(cudaGetLastError());
     }
-    if (a.nlight)
-      SFCI_LAUNCH(c, kl, std::min((a.nlight + LIGHT_WARPS - 1) / LIGHT_WARPS, gl), LIGHT_WARPS * 32, sml, a);
+    if (a.nlight) {
+      kl<<<std::min((a.nlight + LIGHT_WARPS - 1) / LIGHT_WARPS, gl), LIGHT_WARPS * 32, sml, small>>>(a);
+      c.launches++;
+      SFCI_CUDA(cudaGetLastError());
+    }
+    if (both) {
+      if ((st = side.end())) return st;
+      side.join();
+    }
     // survivors, distinct, <v|Hv>, flags, redo count in one read
     u64* rb = (u64*)scratch_get(c, "rw_tot2", 64 * 8);
     SFCI_CUDA(cudaMemcpyAsync(rb, scount, 4 * 8, cudaMemcpyDeviceToDevice, c.stream));

@@ -1,5 +1,5 @@
 """Key sort and magnitude selection on a GB300 through the vector calls, at the
-edges of their warps, slices and of the single-launch form (4,194,304 entries):
+edges of their warps, slices and of the single-launch sort (6,291,456 entries):
 keys and amplitudes must come out exactly as numpy's stable sorts give them."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ from sfci_gb300 import fcidump as fd
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [2, 31, 33, 1023, 1024, 1025, 5000, 152 * 1024, 152 * 1024 + 1, 700001, (1 << 22) + 1]
+SIZES = [2, 31, 33, 1023, 1024, 1025, 5000, 152 * 1024, 152 * 1024 + 1, 700001, (6 << 20) + 1]
 
 
 @pytest.fixture(scope="module")
