@@ -76,6 +76,7 @@ constexpr uint32_t IA_BYTES = TILE * IKC * 2;        // 8192: a 128 x 32 input c
 constexpr uint32_t ISTAGE = IB_BYTES + IA_BYTES;
 constexpr int ISTAGES = 6;
 constexpr int ROW_THREADS = 256;                     // inference: 8 row warps, two per row quarter of TMEM lanes
+constexpr int ICHB = 2;                             // layer-1 chunks per barrier of the row warps
 constexpr int INF_THREADS = ROW_THREADS + 32;        // and one copy warp
 
 }  // namespace mlp
@@ -622,6 +623,14 @@ __global__ void __launch_bounds__(256) k_screen_classify(FwdArgs a, u64 wbeg, u6
 // column halves added through shared memory.  The same function as the
 // training forward (layer1_row), summed in another order.
 //
+// A tile's layer-2 MMAs and the next tile's layer-1 MMAs are issued back to back,
+// and the layer-3 epilogue runs behind them: with each tile's stages in sequence
+// the tensor cores waited for every epilogue.  ICHB input chunks are written per
+// barrier.  2.8e6 groups (1,500 sources of 56 spin orbitals): 2.76 ms before, 2.19
+// ms now (2.31 with one chunk per barrier, 2.19 with four, 2.22 with sixteen row
+// warps); what is left is the 384 KB of chunks a tile streams from L2 through six
+// stages (about 4.3 TB/s over the SMs) and the epilogues.
+//
 // Barrier phases: chunk g of the CTA's sequence uses stage g % 6; its use
 // u = g / 6 completes `full` (copy landed) and, after the MMAs that read the
 // stage, `freed` (tcgen05.commit), both with parity u & 1.  The row warps sync
@@ -654,7 +663,7 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
   float* sb2 = slv + HID;                                               // [256]
   float* sw3 = sb2 + HID;                                               // [256]
   float* slog = sw3 + HID;                                              // [128] second-half logits
-  __shared__ __align__(8) uint64_t bar_full[ISTAGES], bar_free[ISTAGES], bar_done, bar_fin;
+  __shared__ __align__(8) uint64_t bar_full[ISTAGES], bar_free[ISTAGES], bar_done, bar_done2, bar_fin;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -664,6 +673,7 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
       umma::mbar_init(&bar_free[i], 1);
     }
     umma::mbar_init(&bar_done, 1);
+    umma::mbar_init(&bar_done2, 1);
     umma::mbar_init(&bar_fin, 1);
     umma::fence_mbar_init();
     s_fail = 0;
@@ -716,79 +726,104 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
     const int N = a.x.N;
     const u64 nmask0 = N >= 64 ? ~0ull : ((1ull << N) - 1ull);
     const u64 nmask1 = N >= 128 ? ~0ull : (N > 64 ? ((1ull << (N - 64)) - 1ull) : 0ull);
-    for (unsigned t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-      // row `row` of the tile: an entry of the network's list (example, source)
+    // a tile's row of this thread: an entry of the network's list (example, source)
+    struct Row {
+      u64 e, j, occ0, occ1;
+      Feat f;
+      bool valid;
+    };
+    auto load_row = [&](unsigned t) {
+      Row r{};
       const u64 idx = (u64)t * TILE + row;
-      const bool valid = idx < a.nlist;
-      u64 e = 0, j = 0;
-      Feat f{};
-      u64 occ[2] = {0ull, 0ull};
-      if (valid) {
-        e = __ldg(a.list_e + idx);
-        j = __ldg(a.list_j + idx);
-        f = unpack_feat(__ldg(a.list_f + idx));  // computed by the pre-pass
-        const KT key = load_key<KT>(a.x.keys, j);
-        occ[0] = kword(key, 0) & nmask0;
-        if (sizeof(KT) > 8) occ[1] = kword(key, 1) & nmask1;
+      r.valid = idx < a.nlist;
+      if (r.valid) {
+        r.e = __ldg(a.list_e + idx);
+        r.j = __ldg(a.list_j + idx);
+        r.f = unpack_feat(__ldg(a.list_f + idx));  // computed by the pre-pass
+        const KT key = load_key<KT>(a.x.keys, r.j);
+        r.occ0 = kword(key, 0) & nmask0;
+        if (sizeof(KT) > 8) r.occ1 = kword(key, 1) & nmask1;
       }
-      // ---- layer 1, one-hot part: NCH1 chunks
-      for (int c = 0; c < NCH1; ++c, ++g) {
-        const uint32_t st = g % ISTAGES, use = g / ISTAGES;
-        uint8_t* sB = sStg + st * ISTAGE;
-        uint8_t* sX = sB + IB_BYTES;
-        if (use > 0 && !umma::mbar_wait(&bar_free[st], (use - 1) & 1u)) fail = true;
-        // this row's 32 inputs of chunk c: occupancy bits (c < 4), then p, q or r
-        // as a one-hot index; each of the row's two threads writes 16 of them
-        unsigned bits = 0;
-        if (valid) {
-          if (c < 4) {
-            bits = (unsigned)(occ[c >> 1] >> (32 * (c & 1)));
-          } else {
-            const int cc = c - 4;
-            const int oh = cc < 4 ? f.p : (cc < 8 ? f.q : f.r);
-            const int lo = IKC * (cc & 3);
-            if (oh >= lo && oh < lo + IKC) bits = 1u << (oh - lo);
+      return r;
+    };
+    // layer 1, one-hot part: NCH1 chunks, ICHB of them written per barrier; true
+    // when a wait of any row thread failed
+    auto layer1 = [&](const Row& r) -> bool {
+      for (int c0 = 0; c0 < NCH1; c0 += ICHB, g += ICHB) {
+#pragma unroll
+        for (int b = 0; b < ICHB; ++b) {
+          const int c = c0 + b;
+          const uint32_t st = (g + b) % ISTAGES, use = (g + b) / ISTAGES;
+          uint8_t* sX = sStg + st * ISTAGE + IB_BYTES;
+          if (use > 0 && !umma::mbar_wait(&bar_free[st], (use - 1) & 1u)) fail = true;
+          // this row's 32 inputs of chunk c: occupancy bits (c < 4), then p, q or r
+          // as a one-hot index; each of the row's two threads writes 16 of them
+          unsigned bits = 0;
+          if (r.valid) {
+            if (c < 4) {
+              bits = (unsigned)((c >> 1 ? r.occ1 : r.occ0) >> (32 * (c & 1)));
+            } else {
+              const int cc = c - 4;
+              const int oh = cc < 4 ? r.f.p : (cc < 8 ? r.f.q : r.f.r);
+              const int lo = IKC * (cc & 3);
+              if (oh >= lo && oh < lo + IKC) bits = 1u << (oh - lo);
+            }
           }
-        }
 #pragma unroll
-        for (int qq = 0; qq < IKC / 16; ++qq) {
-          const int q = 2 * half + qq;
-          const unsigned by = (bits >> (8 * q)) & 0xffu;
-          uint32_t w[4];
+          for (int qq = 0; qq < IKC / 16; ++qq) {
+            const int q = 2 * half + qq;
+            const unsigned by = (bits >> (8 * q)) & 0xffu;
+            uint32_t w[4];
 #pragma unroll
-          for (int h = 0; h < 4; ++h)
-            w[h] = ((by >> (2 * h)) & 1u ? ONE : 0u) | (((by >> (2 * h + 1)) & 1u ? ONE : 0u) << 16);
-          *reinterpret_cast<uint4*>(sX + umma::tile_offset(row, 8 * q, IKC)) = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int h = 0; h < 4; ++h)
+              w[h] = ((by >> (2 * h)) & 1u ? ONE : 0u) | (((by >> (2 * h + 1)) & 1u ? ONE : 0u) << 16);
+            *reinterpret_cast<uint4*>(sX + umma::tile_offset(row, 8 * q, IKC)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
         }
         umma::fence_async_smem();
         umma::tc_fence_before();
-        if (rows_or(fail)) {
-          fail = true;
-          break;
-        }
+        if (rows_or(fail)) return true;
         if (tid == 0) {
           umma::tc_fence_after();
-          if (umma::mbar_wait(&bar_full[st], use & 1u))
-            umma::gemm_tile(tmem, umma::smem_u32(sX), umma::smem_u32(sB), IKC, idesc, c > 0);
-          else
-            fail = true;
-          umma::mma_commit(&bar_free[st]);
-          if (c == NCH1 - 1) umma::mma_commit(&bar_done);
+#pragma unroll
+          for (int b = 0; b < ICHB; ++b) {
+            const uint32_t st = (g + b) % ISTAGES, use = (g + b) / ISTAGES;
+            uint8_t* sB = sStg + st * ISTAGE;
+            if (!fail && umma::mbar_wait(&bar_full[st], use & 1u))
+              umma::gemm_tile(tmem, umma::smem_u32(sB + IB_BYTES), umma::smem_u32(sB), IKC, idesc, c0 + b > 0);
+            else
+              fail = true;
+            umma::mma_commit(&bar_free[st]);
+          }
+          if (c0 + ICHB == NCH1) umma::mma_commit(&bar_done);
         }
       }
+      return false;
+    };
+    unsigned t = blockIdx.x;
+    Row cur{};
+    if (t < a.ntiles) {
+      cur = load_row(t);
+      if (layer1(cur)) fail = true;
+    }
+    for (; t < a.ntiles; t += gridDim.x) {
+      const unsigned tn = t + gridDim.x;
+      Row nxt{};
+      if (tn < a.ntiles) nxt = load_row(tn);  // in flight during this tile's first epilogue
       if (rows_or(fail)) {
         fail = true;
         break;
       }
       // ---- layer-1 epilogue, this thread's 128 columns
       if (!umma::mbar_wait(&bar_done, done_phase)) fail = true;
-      done_phase ^= 1u;
       if (rows_or(fail)) {
         fail = true;
         break;
       }
       umma::tc_fence_after();
       {
+        const Feat& f = cur.f;
+        const bool valid = cur.valid;
         const float* u = sb1;
         const float* rc = scls + (valid ? f.cls : 0) * HID;
         for (int k = 0; k < HID / 64; ++k) {
@@ -832,10 +867,17 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
           }
           umma::mma_commit(&bar_free[st]);
         }
-        umma::mma_commit(&bar_done);
+        umma::mma_commit(&bar_done2);
       }
       g += NCH2;
-      if (!umma::mbar_wait(&bar_done, done_phase)) fail = true;
+      // ---- the next tile's layer 1 goes to the tensor cores behind this layer 2 (its
+      // accumulator, columns 0..255, was read above), so that it runs during the
+      // epilogue below
+      if (tn < a.ntiles && layer1(nxt)) {
+        fail = true;
+        break;
+      }
+      if (!umma::mbar_wait(&bar_done2, done_phase)) fail = true;
       done_phase ^= 1u;
       if (rows_or(fail)) {
         fail = true;
@@ -852,8 +894,11 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
         for (int i = 0; i < 32; ++i) logit += fmaxf(z[i] + sb2[cb + i], 0.f) * sw3[cb + i];
       }
       if (half) slog[row] = logit;
+      umma::tc_fence_before();
       rows_sync();
       if (!half) {
+        const u64 e = cur.e, j = cur.j;
+        const bool valid = cur.valid;
         logit += slog[row] + b3;
         const float p = 1.f / (1.f + __expf(-logit));
         const bool kept = valid && p >= a.thr;
@@ -861,7 +906,7 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
         if (valid && a.prob) a.prob[e] = p;
         const u64 jj = valid ? j : ~0ull;
         const unsigned same = __match_any_sync(0xffffffffu, jj);
-        const unsigned nt = kept ? f.gsize : 0u, ng = kept ? 1u : 0u;
+        const unsigned nt = kept ? cur.f.gsize : 0u, ng = kept ? 1u : 0u;
         if (same == 0xffffffffu) {
           const unsigned sm_ = warp_sum(nt), sg = warp_sum(ng);
           if (lane == 0 && valid && sm_) {
@@ -873,9 +918,10 @@ __global__ void __launch_bounds__(INF_THREADS, 1) k_mlp_infer(FwdArgs a) {
           atomicAdd(a.kept_groups + j, (u64)ng);
         }
       }
-      umma::tc_fence_before();
-      rows_sync();  // the operand, the logits and TMEM are rewritten by the next tile
+      // the operand, the logits and TMEM are rewritten by the next tile only after
+      // its own barriers
       umma::tc_fence_after();
+      cur = nxt;
     }
     if (fail) {
       s_fail = 1;  // stops the copy warp
