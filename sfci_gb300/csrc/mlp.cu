@@ -626,10 +626,10 @@ __global__ void __launch_bounds__(256) k_screen_classify(FwdArgs a, u64 wbeg, u6
 // A tile's layer-2 MMAs and the next tile's layer-1 MMAs are issued back to back,
 // and the layer-3 epilogue runs behind them: with each tile's stages in sequence
 // the tensor cores waited for every epilogue.  ICHB input chunks are written per
-// barrier.  2.8e6 groups (1,500 sources of 56 spin orbitals): 2.76 ms before, 2.19
-// ms now (2.31 with one chunk per barrier, 2.19 with four, 2.22 with sixteen row
-// warps); what is left is the 384 KB of chunks a tile streams from L2 through six
-// stages (about 4.3 TB/s over the SMs) and the epilogues.
+// barrier.  A predict call without probabilities on 1,500 sources of 56 spin
+// orbitals (2.8e6 groups), host time: 2.76 ms before, 2.19 ms now (2.31 with one
+// chunk per barrier, 2.19 with four, 2.22 with sixteen row warps).  A tile streams
+// 24 chunks of 16 KB: by arithmetic 8.6 GB over the call, not a profiled rate.
 //
 // Barrier phases: chunk g of the CTA's sequence uses stage g % 6; its use
 // u = g / 6 completes `full` (copy landed) and, after the MMAs that read the
