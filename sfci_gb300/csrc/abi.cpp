@@ -71,6 +71,18 @@ void scratch_release(Ctx& c, const char* name) {
   c.scratch.erase(it);
 }
 
+void scratch_release_lists(Ctx& c) {
+  cudaStreamSynchronize(c.stream);
+  for (auto it = c.scratch.begin(); it != c.scratch.end();) {
+    if (it->first.compare(0, 3, "rw_") && it->first.compare(0, 3, "pr_")) {
+      ++it;
+      continue;
+    }
+    if (it->second.p) cudaFree(it->second.p);
+    it = c.scratch.erase(it);
+  }
+}
+
 void scratch_release_plan(Ctx& c) {
   for (const char* nm : {"sp_l1k", "sp_l1a", "sp_l2k", "sp_l2a", "sp_sk", "sp_sa", "rs_keys", "rs_vals", "topk_k",
                          "topk_a"})

@@ -111,6 +111,7 @@ void scratch_free_all(Ctx& c);
 // re-plans from the memory that is then free)
 void scratch_release(Ctx& c, const char* name);
 void scratch_release_plan(Ctx& c);
+void scratch_release_lists(Ctx& c);  // the row product's and the pair search's lists
 // pinned host words for readbacks
 u64* pinned_words(Ctx& c, size_t n);
 

@@ -1648,6 +1648,12 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
   {
     size_t freeb = 0, totb = 0;
     SFCI_CUDA(cudaMemGetInfo(&freeb, &totb));
+    // the row product's and the pair search's lists make way for a plan that cannot
+    // hold every term at both levels beside them
+    if ((double)freeb * 0.85 < 3.0 * (double)T * tb + ((size_t)256 << 20)) {
+      scratch_release_lists(c);
+      SFCI_CUDA(cudaMemGetInfo(&freeb, &totb));
+    }
     // the plan's buffers (replaced in place when they grow): the two term
     // levels and the survivors; the plan also leaves room for the sort scratch
     // the survivors go through (not counted here: whatever it holds stays held)
