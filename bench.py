@@ -452,6 +452,11 @@ def _finish_gpu(args, rank, ws, dist, ctx, sysd, path, nd, M, NE, W, n_in, C, T_
     L1_BITS, DIGIT_BITS = 9, 9
     b = max(1, int(round(np.log2(max(stats["leaves"], 1)))))
     levels = -(-(b - min(b, L1_BITS)) // DIGIT_BITS)
+    # the row form generates and merges in one kernel and stores no term: "leaves"
+    # are its work units, and it has no generation or partition phase
+    rows = prof["scatter"][1] == 0 and prof["partition"][1] == 0 and prof["merge"][1] > 0
+    if rows:
+        levels = 0
     # algorithmic bytes per phase (all launches of the timed steps)
     alg = {
         "scatter": tbytes * T * args.steps,                      # generated (key, amp) terms written once
@@ -464,6 +469,9 @@ def _finish_gpu(args, rank, ws, dist, ctx, sysd, path, nd, M, NE, W, n_in, C, T_
     }
     kernels = {"scatter": "k_gen<SCATTER>", "partition": "k_part<COUNT,SCATTER>", "merge": "k_leafw",
                "count": "k_gen<COUNT>", "select": "select_threshold", "sort": "radix_sort_pairs", "other": "-"}
+    if rows:
+        alg["merge"] = tbytes * (n_in + surv) * args.steps  # sources read, survivors written
+        kernels.update(merge="k_rows_cta", count="row tables (k_rows_*)")
     # DRAM bytes per generated term measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum over
     # the launches of one 56-orbital Nd=1e4 SpMSpV in one generation pass, 2 partition levels, 8 GB device
     # budget: level buffers well above L2), scaled here to a launch by the terms it processes
@@ -473,7 +481,7 @@ def _finish_gpu(args, rank, ws, dist, ctx, sysd, path, nd, M, NE, W, n_in, C, T_
     per_launch_bytes = alg[dom] / max(dl, 1)
     per_launch_ms = dms / max(dl, 1)
     achieved = per_launch_bytes / (per_launch_ms * 1e-3) / 1e9 if per_launch_ms > 0 else 0.0
-    traffic = (ncu_bytes_per_term[dom] * T * args.steps / max(dl, 1)) if (dom in ncu_bytes_per_term and W == 1) \
+    traffic = (ncu_bytes_per_term[dom] * T * args.steps / max(dl, 1)) if (dom in ncu_bytes_per_term and W == 1 and not rows) \
         else None  # measured for one-word keys
     value = T_conn * ws / (ms_max * 1e-3)
     e2e_val = T_conn * ws / e2e_s if e2e_s else None
@@ -492,7 +500,7 @@ def _finish_gpu(args, rank, ws, dist, ctx, sysd, path, nd, M, NE, W, n_in, C, T_
                   "survivors_per_step": surv, "output_dets": out_len, "passes": stats["passes"],
                   "leaves": stats["leaves"], "partition_levels": levels,
                   "terms_gb_per_step": tbytes * T / 1e9},
-        "roofline": {"bound": "hbm", "kernel": kernels[dom], "phase": dom, "achieved": achieved, "peak": hbm,
+        "roofline": {"bound": "issue" if rows and dom == "merge" else "hbm", "kernel": kernels[dom], "phase": dom, "achieved": achieved, "peak": hbm,
                      "unit": "GB/s", "frac": achieved / hbm, "peak_source": how, "traffic": traffic,
                      "traffic_unit": "bytes per launch", "algorithmic_bytes_per_launch": per_launch_bytes,
                      "launches": dl, "ms_per_launch": per_launch_ms},
