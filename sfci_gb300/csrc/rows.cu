@@ -799,13 +799,14 @@ __host__ __device__ inline size_t row_cta_smem(unsigned smax) {
   return row_table_bytes<typename StrOf<W>::T>(1u << TB) + rows_al16(sizeof(unsigned) * (smax + 1)) * 7;
 }
 
-// Larger rows: a CTA per unit.  Bound by instruction issue (about 190 instructions
-// a term: hash, two-word rounding, three or four 32-bit shared reductions); DRAM
-// is idle and L2 serves the lists.  The whole product with 120,000 sources of 56
-// spin orbitals (3.7e9 terms) takes 74 ms against 179 ms in the partitioned
-// pipeline, 3,001 sources 3.5 against 5.7 ms, 9,001 of 68 spin orbitals 22 against
-// 37 ms.  The unit's range of H is walked in steps that fill
-// the table to about half; a step whose table overflows is redone at half its
+// Larger rows: a CTA per unit.  Bound by instruction issue (12.5 warp instructions
+// a term at 23 of 32 lanes, 0.61e9 terms from 20,000 sources of 56 spin orbitals:
+// hash, two-word rounding, three or four 32-bit shared reductions, and the steps'
+// set-up); DRAM is idle and L2 serves the lists.  Whole calls with the result's
+// download, partitioned pipeline against this one: 120,000 sources of 56 spin
+// orbitals (3.7e9 terms) 178.5 and 63.4 ms, 3,001 sources 5.7 and 3.2 ms, 9,001 of
+// 68 spin orbitals 37.2 and 21.9 ms.  The unit's range of H is walked in steps
+// that fill the table to LOAD; a step whose table overflows is redone at half its
 // width.
 template <int W, int DB, int NT, int TB_MAX>
 __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(RowArgs<W> a) {
