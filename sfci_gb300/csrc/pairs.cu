@@ -71,17 +71,21 @@ struct PairArgs {
   const double* diagE;  // by key index
   double lambda;
   const double* bamps;  // ENERGY: of the bras
-  u64* esum;            // ENERGY: exact 128-bit sum
+  u64* esum;            // ENERGY: exact 128-bit sum of the products times 4^up
+  int up;               // ENERGY: power of two that brings the largest amplitude into [1, 2)
   u64 *plo, *phi;       // PROJECT: exact sums by bra index (split form)
 };
 
 template <int W>
-__global__ void k_pair_rank(Side<W> s, int na, int nb, int N, const unsigned* bin, unsigned* flag) {
+__global__ void k_pair_rank(Side<W> s, int na, int nb, int N, const unsigned* bin, unsigned* flag,
+                            const double* __restrict__ amps, u64* __restrict__ amax) {
   typedef typename StrOf<W>::T ST;
   typedef typename KeyOf<W>::T KT;
   unsigned bad = 0;
+  u64 mx = 0;  // largest |amplitude|, as an integer
   for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < s.n; j += (u64)gridDim.x * blockDim.x) {
     const KT k = s.keys[j];
+    if (amps) mx = max(mx, abs_bits(amps[j]));
     if (s.table && key_eq(k, key_empty<KT>())) {
       s.ra[j] = ~0u;
       continue;
@@ -97,6 +101,11 @@ __global__ void k_pair_rank(Side<W> s, int na, int nb, int N, const unsigned* bi
     atomicAdd((unsigned*)(s.arank + r), 1u);
   }
   if (bad) atomicOr(flag, 1u);
+  if (amps) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0 && mx) atomicMax((unsigned long long*)amax, (unsigned long long)mx);
+  }
 }
 
 template <int W>
@@ -212,8 +221,10 @@ __global__ void __launch_bounds__(256) k_pair_nbrs(PairArgs<W> a, unsigned nslic
 }
 
 // A warp per ket.  Sums over the pairs found are exact (ENERGY: 128-bit sum of
-// each product c_bra * term rounded once to the FX_FRAC grid; PROJECT: the bras'
-// merge accumulators), so they do not depend on the order.
+// each product c_bra * term rounded once to the FX_FRAC grid of the vector scaled to
+// a largest amplitude in [1, 2), so that the energy of a vector times a power of
+// two has the same bits; PROJECT: the bras' merge accumulators), so they do not
+// depend on the order.
 template <int W, bool ENERGY>
 __global__ void __launch_bounds__(256) k_pairs(PairArgs<W> a) {
   typedef typename StrOf<W>::T ST;
@@ -227,7 +238,7 @@ __global__ void __launch_bounds__(256) k_pairs(PairArgs<W> a) {
     amp = signed_by(par ^ (x >> 31), amp);
     if (ENERGY) {
       u64 l, h;
-      fx128_of(amp * a.bamps[x & 0x7fffffffu], l, h, bad);
+      fx128_of(amp * a.bamps[x & 0x7fffffffu], l, h, bad, a.up);
       slo += l;
       shi += h + (slo < l ? 1ull : 0ull);
     } else {
@@ -240,7 +251,8 @@ __global__ void __launch_bounds__(256) k_pairs(PairArgs<W> a) {
   for (u64 p = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < k.n; p += nw) {
     const unsigned g = k.pg[p], x = k.px[p];
     const ST A = k.gstr[g], H = k.pH[p], B = hs_inv(H);
-    const double c0 = a.amps[x & 0x7fffffffu], c = signed_by(x >> 31, c0);
+    const double c0 = ENERGY ? scalbn(a.amps[x & 0x7fffffffu], a.up) : a.amps[x & 0x7fffffffu];
+    const double c = signed_by(x >> 31, c0);
     const u64 o0 = a.noff[g], o1 = a.noff[g + 1];
     // groups one move away
     for (unsigned i0 = (unsigned)o0; i0 < (unsigned)o1; i0 += 32) {
@@ -331,12 +343,14 @@ struct Builder {
     return (unsigned)std::max<u64>(1, std::min<u64>((n + per - 1) / per, gmax));
   }
   // ranks and the scanned rank table
-  int rank(Side<W>& s, const std::string& p, unsigned RA, int na, int nb, const unsigned* bin, unsigned* flag) {
+  // (amps: their largest magnitude goes to *amax)
+  int rank(Side<W>& s, const std::string& p, unsigned RA, int na, int nb, const unsigned* bin, unsigned* flag,
+           const double* amps = nullptr, u64* amax = nullptr) {
     s.ra = (unsigned*)get(p + "ra", s.n * 4);
     s.arank = (u64*)get(p + "arank", ((u64)RA + 1) * 8);
     if (!ok) return SFCI_OK;
     SFCI_CUDA(cudaMemsetAsync(s.arank, 0, ((u64)RA + 1) * 8, c.stream));
-    SFCI_LAUNCH(c, k_pair_rank<W>, grid(s.n, 256), 256, 0, s, na, nb, c.N, bin, flag);
+    SFCI_LAUNCH(c, k_pair_rank<W>, grid(s.n, 256), 256, 0, s, na, nb, c.N, bin, flag, amps, amax);
     SFCI_LAUNCH(c, k_rows_mark, grid(RA, 256), 256, 0, s.arank, RA);
     return scan_excl(c, s.arank, s.arank, RA);
   }
@@ -410,7 +424,7 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   a.ntest = tot + 5;
   a.diagE = diagE;
   SFCI_CUDA(cudaMemsetAsync(tot, 0, 8 * 8, c.stream));
-  if ((st = b.rank(a.bra, "pr_b", a.RA, na, nb, a.bin, a.flag)) || !b.ok) return st;
+  if ((st = b.rank(a.bra, "pr_b", a.RA, na, nb, a.bin, a.flag, a.bamps, tot + 3)) || !b.ok) return st;
   if (ENERGY) {
     a.ket = a.bra;
   } else if ((st = b.rank(a.ket, "pr_k", a.RA, na, nb, a.bin, a.flag)) || !b.ok) {
@@ -421,6 +435,10 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   u64 th[5], rb[6];
   if ((st = read_words(c, tot, sizeof th, th))) return st;
   if ((unsigned)th[4]) return SFCI_OK;
+  // (subnormal largest amplitudes: the energy is zero; not finite: no scaling, and
+  // the sum reports it)
+  const int emax = (int)(th[3] >> 52);
+  if (ENERGY && emax < 0x7ff) a.up = std::min(1022, 1023 - emax);
   a.bra.nG = (unsigned)(th[0] >> 32);
   a.ket.nG = (unsigned)(th[1] >> 32);
   if (a.ket.nG * nda >= (1ull << 32)) return SFCI_OK;
@@ -475,7 +493,7 @@ int pairs_energy(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   if (st || !*done) return st;
   u64 s[2];
   if ((st = read_words(c, a.esum, sizeof s, s))) return st;
-  *E = fx_to_double(s[0], s[1]);
+  *E = std::ldexp(fx_to_double(s[0], s[1]), -2 * a.up);
   *terms = n * det_terms(a.na, a.nva, a.nb, c.M - a.nb);
   return SFCI_OK;
 }
