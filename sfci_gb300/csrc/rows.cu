@@ -105,7 +105,7 @@ struct RowArgs {
   u64* arank;            // per alpha rank: sources | 1 << 32 when any, then their exclusive scan
   uint32_t* brank;       // per beta rank: 1 when any, then the exclusive scan
   unsigned RA, RB;
-  unsigned* flag;        // [0] not eligible, [1] term too large, [2] largest group
+  unsigned* flag;        // [0] not eligible, [1] a row's term too large, [2] largest group
   // groups (distinct alpha strings), in rank order
   unsigned nG, nB;
   ST* gstr;
@@ -164,6 +164,11 @@ struct RowArgs {
   int max_exp;           // terms are below 2^max_exp
 };
 
+// a term the accumulators do not take: at least 2^max_exp, or not finite
+__device__ __forceinline__ bool term_too_large(double x, int max_exp) {
+  return (int)(abs_bits(x) >> 52) >= 1023 + max_exp;
+}
+
 // opposite-spin integral of the moves i -> a (alpha) and j -> b (beta): the block
 // named by the lower of the two occupied spin orbitals (gen.cuh, term_amp)
 __global__ void k_rows_os(HamView h, double* __restrict__ os) {
@@ -209,7 +214,8 @@ __global__ void k_rows_split(RowArgs<W> a) {
 }
 
 // extra sources: each adds one term to the row of its own alpha string (counts,
-// then entries; an extra determinant of other spin counts declines the product)
+// then entries; an extra determinant of other spin counts, or too large a term,
+// declines the product)
 template <int W, bool FILL>
 __global__ void k_rows_extra(RowArgs<W> a) {
   typedef typename StrOf<W>::T ST;
@@ -218,7 +224,8 @@ __global__ void k_rows_extra(RowArgs<W> a) {
     ST sa, sb;
     split_key(a.keys[a.ns + j], sa, sb);
     if (!FILL) {
-      if (spop(sa) != a.na || spop(sb) != a.nb || !key_within(a.keys[a.ns + j], a.h.N)) {
+      if (spop(sa) != a.na || spop(sb) != a.nb || !key_within(a.keys[a.ns + j], a.h.N) ||
+          term_too_large(a.amps[a.ns + j], a.max_exp)) {
         bad = 1;
         a.xra[j] = ~0u;
         continue;
@@ -424,12 +431,21 @@ __global__ void k_rows_list0(RowArgs<W> a) {
   }
 }
 
+// Diagonal elements.  With H's largest elements on the diagonal, a term out of the
+// accumulators' range is first of all a diagonal one: the product is declined here,
+// before its lists are built.  Found by the rows alone, after their last term, it
+// cost the whole row form: 3,001 sources of 56 spin orbitals, out of range, 9.9 ms,
+// now 6.4, the partitioned pipeline alone 6.3.  A term found by the rows ends them
+// (20,000 sources 27 ms, the rows 18 and the pipeline 23).
 template <int W>
 __global__ void k_rows_diag(RowArgs<W> a, double* __restrict__ diagE) {
   const u64 nw = ((u64)gridDim.x * blockDim.x) >> 5;
   for (u64 w = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < a.ns; w += nw) {
     const double D = diag_element_warp(a.keys[w], a.h);
-    if ((threadIdx.x & 31) == 0) diagE[w] = D;
+    if ((threadIdx.x & 31) == 0) {
+      diagE[w] = D;
+      if (term_too_large((D - a.lambda) * (a.coeff * a.amps[w]), a.max_exp)) atomicOr(a.flag, 1u);
+    }
   }
 }
 
@@ -753,6 +769,8 @@ __global__ void __launch_bounds__(LIGHT_WARPS * 32) k_rows_light(RowArgs<W> a) {
   unsigned bad = 0;
   u64 uq = 0;
   const u64 nw = (u64)gridDim.x * LIGHT_WARPS;
+  // (a term was too large: the product is declined)
+  if (__shfl_sync(0xffffffffu, *(volatile unsigned*)(a.flag + 1), 0)) return;
   for (u64 i = (u64)blockIdx.x * LIGHT_WARPS + warp; i < a.nlight; i += nw) {
     const unsigned r = a.light[i];
     // (a later launch sees the same survivor count, so a skipped row is never half written)
@@ -842,7 +860,8 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
   u64 uq = 0, dlo = 0, dhi = 0;  // distinct targets; this thread's share of <v|Hv>
   for (;;) {
     if (tid == 0) {
-      const unsigned u = atomicAdd(a.ucur, 1u);
+      // (no more units once a term was too large: the product is then declined)
+      const unsigned u = *(volatile unsigned*)(a.flag + 1) ? ~0u : atomicAdd(a.ucur, 1u);
       s_unit = u < a.nunits ? a.units[u] : make_uint4(0u, 1u, 0u, 0u);
     }
     __syncthreads();
@@ -1134,8 +1153,8 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
     }
     __syncthreads();
     if (lo < end && tid == 0) a.redo[atomicAdd(a.nredo, 1u)] = make_uint4(r, (unsigned)lo, (unsigned)(end - 1), 0u);
+    if (bad | dbad) atomicOr(a.flag + 1, 1u);
   }
-  if (bad || dbad) atomicOr(a.flag + 1, 1u);
   // exact 128-bit sum over the CTA, then one global addition
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -1315,6 +1334,9 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.arank = (u64*)get("rw_arank", (RA + 1) * 8);
   a.brank = (uint32_t*)get("rw_brank", (RB + 1) * 4);
   a.flag = (unsigned*)get("rw_flag", 256 * 4);
+  double* diagE = (double*)get("rw_diag", ns * 8);
+  a.diagE = diagE;
+  a.max_exp = d16 ? 15 : 10;
   if (!ok) return SFCI_OK;
   a.bins = a.flag + 8;  // 64 counts, 64 cursors
   a.ucur = a.flag + 144;
@@ -1325,6 +1347,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   const unsigned gmax = (unsigned)c.sm_count * 8;
   auto grid_of = [&](u64 n, unsigned per) { return (unsigned)std::max<u64>(1, std::min<u64>((n + per - 1) / per, gmax)); };
   SFCI_LAUNCH(c, k_rows_split<W>, grid_of(ns, 256), 256, 0, a);
+  SFCI_LAUNCH(c, k_rows_diag<W>, (unsigned)std::max<u64>(1, std::min<u64>((ns + 7) / 8, gmax * 2)), 256, 0, a, diagE);
   SFCI_LAUNCH(c, k_rows_mark, grid_of(RA, 256), 256, 0, a.arank, a.RA);
   if ((st = scan_excl(c, a.arank, a.arank, RA))) return st;
   if ((st = scan_excl_u32(c, a.brank, a.brank, RB))) return st;
@@ -1374,8 +1397,6 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.pc = (double*)get("rw_pc", ns * 8);
   a.pa = (double*)get("rw_pa", ns * 8);
   a.pd = (double*)get("rw_pd", ns * 8);
-  double* diagE = (double*)get("rw_diag", ns * 8);
-  a.diagE = diagE;
   a.c0 = (uint32_t*)get("rw_c0", (nb0max + 1) * 4);
   a.off0 = (uint32_t*)get("rw_off0", (nb0max + 1) * 4);
   a.c1 = (uint32_t*)get("rw_c1", (nb1max + 1) * 4);
@@ -1469,11 +1490,9 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.soft = SC - slack;
   a.cut = fx_cut(c.opts.coeff_cut);
   a.smax = (unsigned)nsa;
-  a.max_exp = d16 ? 15 : 10;
   SFCI_CUDA(cudaMemsetAsync(scount, 0, 4 * 8, c.stream));
   SFCI_CUDA(cudaMemsetAsync(a.c0, 0, (nb0 + 1) * 4, c.stream));
   SFCI_CUDA(cudaMemsetAsync(a.c1, 0, (nb1 + 1) * 4, c.stream));
-  SFCI_LAUNCH(c, k_rows_diag<W>, (unsigned)std::max<u64>(1, std::min<u64>((ns + 7) / 8, gmax * 2)), 256, 0, a, diagE);
   SFCI_LAUNCH(c, (k_rows_list0<W, false>), grid_of(ns, 256), 256, 0, a);
   if ((st = scan_excl_u32(c, a.c0, a.off0, nb0))) return st;
   SFCI_LAUNCH(c, (k_rows_list0<W, true>), grid_of(ns, 256), 256, 0, a);
