@@ -659,7 +659,7 @@ int sfci_vec_upload(sfci_vec* v, const uint64_t* keys, const double* amps, uint6
   int st = SFCI_W(c, sort_vec_impl, c, v->v);
   if (st) return st;
   SFCI_CUDA(cudaStreamSynchronize(c.stream));
-  return SFCI_OK;
+  return coop_check(c);
 }
 
 int sfci_vec_download(const sfci_vec* v, uint64_t* keys, double* amps, uint64_t cap, uint64_t* len) {

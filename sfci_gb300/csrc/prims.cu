@@ -174,7 +174,12 @@ constexpr int CO_DIGIT = 8;
 constexpr int CO_BATCH = 2;  // entries a lane loads ahead
 
 // Grid barrier of a cooperative launch (every CTA is resident): true when all
-// CTAs arrived, false (and *err set) when they did not within the poll limit.
+// CTAs arrived, false (and *err set) when they did not within the poll limit.  The
+// limit, about 40 s, is there so that nothing waits forever: CTAs that get their
+// SMs late, behind another stream's kernel of a few seconds, are waited for.  A CTA
+// that gives up says so in the counter, and every other one leaves with it.
+constexpr unsigned COOP_GAVE_UP = 1u << 31;
+constexpr unsigned COOP_POLLS = 1u << 16, COOP_NAPS = 1u << 24;  // without and with a nap of 2 us between them
 __device__ bool coop_barrier(unsigned* bar, unsigned target, unsigned* err) {
   __shared__ int s_ok;
   __syncthreads();
@@ -182,15 +187,20 @@ __device__ bool coop_barrier(unsigned* bar, unsigned target, unsigned* err) {
     __threadfence();
     atomicAdd(bar, 1u);
     int ok = 0;
-    for (unsigned spin = 0; spin < (1u << 22); ++spin) {
+    for (unsigned spin = 0; spin < COOP_POLLS + COOP_NAPS; ++spin) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if (v & COOP_GAVE_UP) break;
       if (v >= target) {
         ok = 1;
         break;
       }
+      if (spin >= COOP_POLLS) __nanosleep(2000);
     }
-    if (!ok) *(volatile unsigned*)err = 1u;
+    if (!ok) {
+      atomicOr(bar, COOP_GAVE_UP);
+      *(volatile unsigned*)err = 1u;
+    }
     __threadfence();
     s_ok = ok;
   }
