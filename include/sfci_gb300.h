@@ -261,6 +261,12 @@ int sfci_ctx_set_tuning(sfci_ctx* ctx, const int* tuning4);
  * its own terms, or by hash bins, each pass regenerating every term.  Results
  * never depend on the mode. */
 int sfci_ctx_set_class_passes(sfci_ctx* ctx, int mode);
+/* Key sort and magnitude selection as one launch each, whose blocks wait for one
+ * another (1, the default), or as a chain of launches without such a wait (0), which
+ * is also what runs where the GPU cannot hold the one launch's grid.  The results
+ * are the same.  The wait ends after about 40 s, with SFCI_ERR_CUDA from the next
+ * call that reads from the device. */
+int sfci_ctx_set_grid_barrier(sfci_ctx* ctx, int on);
 int sfci_ctx_get_tuning(const sfci_ctx* ctx, int* tuning4);
 int sfci_autotune(sfci_ctx* ctx, const sfci_vec* in, sfci_vec* out, int* best4, double* best_ms);
 

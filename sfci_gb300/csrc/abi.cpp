@@ -421,6 +421,12 @@ int sfci_ctx_set_class_passes(sfci_ctx* x, int mode) {
   return SFCI_OK;
 }
 
+int sfci_ctx_set_grid_barrier(sfci_ctx* x, int on) {
+  if (!x) return set_error(SFCI_ERR_ARG, "null context");
+  x->c.grid_barrier = on != 0;
+  return SFCI_OK;
+}
+
 int sfci_ctx_get_tuning(const sfci_ctx* x, int* t4) {
   if (!x || !t4) return set_error(SFCI_ERR_ARG, "null argument");
   const Ctx& c = x->c;

@@ -69,6 +69,7 @@ struct Ctx {
   // pinned host staging for small readbacks
   u64* h_pin = nullptr;
   size_t h_pin_words = 0;
+  bool grid_barrier = true;    // sort and selection in one launch with a grid barrier (prims.cu)
   unsigned* h_coop = nullptr;  // set by a kernel whose grid barrier ran out of its poll limit
   // batched contexts: one Hamiltonian per instance (device HamView table);
   // ninst = 0 for an ordinary context

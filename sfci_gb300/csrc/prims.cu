@@ -337,6 +337,23 @@ __global__ void __launch_bounds__(CO_THREADS, 1) k_rs_coop(KT* ka, double* va, K
     }
 }
 
+// Cooperative launch; *ran false when the context's one-launch forms are switched
+// off, or when the GPU cannot hold the grid at once (a share of the SMs under MPS, for
+// one): the callers then take the multi-launch forms.
+static int coop_launch(Ctx& c, const void* kern, unsigned G, void** args, size_t sm, bool* ran) {
+  *ran = false;
+  if (!c.grid_barrier) return SFCI_OK;
+  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(CO_THREADS), args, sm, c.stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    return SFCI_OK;
+  }
+  SFCI_CUDA(e);
+  c.launches++;
+  *ran = true;
+  return SFCI_OK;
+}
+
 // entries a CTA takes, for n entries
 static unsigned coop_slice(const Ctx& c, size_t n) {
   const size_t s = (n + c.sm_count - 1) / c.sm_count;
@@ -344,7 +361,7 @@ static unsigned coop_slice(const Ctx& c, size_t n) {
 }
 
 template <int W>
-static int radix_sort_coop(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, int nbits) {
+static int radix_sort_coop(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, int nbits, bool* ran) {
   typedef typename KeyOf<W>::T KT;
   const int nb8 = (nbits + 7) / 8 * 8;  // the bits the 8-bit passes cover
   int passes = (nb8 + CO_DIGIT - 1) / CO_DIGIT, bits = (nb8 + passes - 1) / passes;
@@ -363,9 +380,7 @@ static int radix_sort_coop(Ctx& c, typename KeyOf<W>::T* keys, double* vals, siz
   SFCI_CUDA(cudaFuncSetAttribute(k_rs_coop<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(uint32_t) * ((size_t)(CO_WARPS + 1) << CO_DIGIT))));
   void* args[] = {&keys, &vals, &k2, &v2, &un, &slice, &passes, &bits, &cm, &bar, &err};
-  SFCI_CUDA(cudaLaunchCooperativeKernel((const void*)k_rs_coop<KT>, dim3(G), dim3(CO_THREADS), args, sm, c.stream));
-  c.launches++;
-  return SFCI_OK;
+  return coop_launch(c, (const void*)k_rs_coop<KT>, G, args, sm, ran);
 }
 
 template <int W>
@@ -373,7 +388,9 @@ int radix_sort_pairs(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n,
   typedef typename KeyOf<W>::T KT;
   if (n <= 1 || nbits <= 0) return SFCI_OK;
   if (n >= (1ull << 32)) return set_error(SFCI_ERR_UNSUPPORTED, "radix sort beyond 2^32 items");
-  if (n <= COOP_MAX) return radix_sort_coop<W>(c, keys, vals, n, nbits);
+  bool ran = false;
+  int st;
+  if (n <= COOP_MAX && ((st = radix_sort_coop<W>(c, keys, vals, n, nbits, &ran)) || ran)) return st;
   size_t ntiles = (n + RS_TILE - 1) / RS_TILE;
   KT* k2 = (KT*)scratch_get(c, "rs_keys", n * sizeof(KT));
   double* v2 = (double*)scratch_get(c, "rs_vals", n * sizeof(double));
@@ -788,10 +805,10 @@ __global__ void __launch_bounds__(CO_THREADS, 1) k_sel_coop(SelArgs s, const KT*
 }
 
 // mode 0: entries with bits above low_key; 1: the k largest first; 2: the same with
-// every entry tied with the k-th (0 < k < n)
+// every entry tied with the k-th (0 < k < n); *ran false: not done (coop_launch)
 template <int W>
 static int select_coop(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, int mode, size_t k,
-                       long long low_key, typename KeyOf<W>::T* ok, double* oa, size_t* m) {
+                       long long low_key, typename KeyOf<W>::T* ok, double* oa, size_t* m, bool* ran) {
   typedef typename KeyOf<W>::T KT;
   const size_t words = 6 * 4096 + 2 * (size_t)c.sm_count + 8;
   uint32_t* buf = (uint32_t*)scratch_get(c, "sel_coop", words * sizeof(uint32_t));
@@ -815,11 +832,10 @@ static int select_coop(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia,
   SFCI_CUDA(cudaFuncSetAttribute(k_sel_coop<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(SEL_COPIES * 4096 * sizeof(uint32_t))));
   void* args[] = {&s, &ik, &ok, &oa};
-  SFCI_CUDA(cudaLaunchCooperativeKernel((const void*)k_sel_coop<KT>, dim3(G), dim3(CO_THREADS), args, sm, c.stream));
-  c.launches++;
+  int st = coop_launch(c, (const void*)k_sel_coop<KT>, G, args, sm, ran);
+  if (st || !*ran) return st;
   u64 got = 0;
-  int st = read_words(c, s.m, sizeof(u64), &got);
-  if (st) return st;
+  if ((st = read_words(c, s.m, sizeof(u64), &got))) return st;
   *m = (size_t)got;
   return SFCI_OK;
 }
@@ -834,7 +850,9 @@ int compact_top(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t
 template <int W>
 int compact_cut(Ctx& c, const typename KeyOf<W>::T* ik, const double* ia, size_t n, double cut,
                 typename KeyOf<W>::T* ok, double* oa, size_t* m) {
-  if (n && n <= SEL_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(cut), ok, oa, m);
+  bool ran = false;
+  int st;
+  if (n && n <= SEL_MAX && ((st = select_coop<W>(c, ik, ia, n, 0, 0, cut_key(cut), ok, oa, m, &ran)) || ran)) return st;
   KeepRule r{0, 0, 0, cut_key(cut), -1ll};
   return compact_rule<W>(c, ik, ia, n, r, ok, oa, m);
 }
@@ -843,10 +861,13 @@ template <int W>
 int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t k, double tiny,
                  typename KeyOf<W>::T* ok, double* oa, size_t* m) {
   typedef typename KeyOf<W>::T KT;
+  bool ran = false;
+  int st;
   if (n <= k) {
     if (tiny >= 0.0) {
       // filter only: keep |a| > tiny (all of them pass the selection)
-      if (n && n <= SEL_MAX) return select_coop<W>(c, ik, ia, n, 0, 0, cut_key(tiny), ok, oa, m);
+      if (n && n <= SEL_MAX && ((st = select_coop<W>(c, ik, ia, n, 0, 0, cut_key(tiny), ok, oa, m, &ran)) || ran))
+        return st;
       // tau = 0 keeping all n ties keeps everything before the tiny filter
       KeepRule r{1, 0ull, (u64)n, -1ll, cut_key(tiny)};
       return compact_rule<W>(c, ik, ia, n, r, ok, oa, m);
@@ -858,32 +879,26 @@ int top_k_stable(Ctx& c, typename KeyOf<W>::T* ik, double* ia, size_t n, size_t 
     *m = n;
     return SFCI_OK;
   }
-  int st;
-  if (n <= SEL_MAX && k > 0) {
-    if (ok != ik) return select_coop<W>(c, ik, ia, n, 1, k, cut_key(tiny), ok, oa, m);
-    KT* tk = (KT*)scratch_get(c, "topk_k", n * sizeof(KT));
-    double* ta = (double*)scratch_get(c, "topk_a", n * sizeof(double));
-    if (!tk || !ta) return SFCI_ERR_NOMEM;
-    if ((st = select_coop<W>(c, ik, ia, n, 1, k, cut_key(tiny), tk, ta, m))) return st;
-    SFCI_CUDA(cudaMemcpyAsync(ok, tk, *m * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
-    SFCI_CUDA(cudaMemcpyAsync(oa, ta, *m * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-    return SFCI_OK;
-  }
-  u64 tau;
-  size_t gt;
-  if ((st = select_threshold(c, ia, n, k, &tau, &gt))) return st;
-  size_t need_eq = k - gt;
+  // a compaction may not run in place across tiles: it is staged through scratch
+  KT* tk = ok;
+  double* ta = oa;
   if (ok == ik) {
-    // compaction may not run in place across tiles; stage through scratch
-    KT* tk = (KT*)scratch_get(c, "topk_k", n * sizeof(KT));
-    double* ta = (double*)scratch_get(c, "topk_a", n * sizeof(double));
+    tk = (KT*)scratch_get(c, "topk_k", n * sizeof(KT));
+    ta = (double*)scratch_get(c, "topk_a", n * sizeof(double));
     if (!tk || !ta) return SFCI_ERR_NOMEM;
-    if ((st = compact_top<W>(c, ik, ia, n, tau, need_eq, tiny, tk, ta, m))) return st;
+  }
+  if (n <= SEL_MAX && k > 0 && (st = select_coop<W>(c, ik, ia, n, 1, k, cut_key(tiny), tk, ta, m, &ran))) return st;
+  if (!ran) {
+    u64 tau;
+    size_t gt;
+    if ((st = select_threshold(c, ia, n, k, &tau, &gt))) return st;
+    if ((st = compact_top<W>(c, ik, ia, n, tau, k - gt, tiny, tk, ta, m))) return st;
+  }
+  if (ok == ik) {
     SFCI_CUDA(cudaMemcpyAsync(ok, tk, *m * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
     SFCI_CUDA(cudaMemcpyAsync(oa, ta, *m * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-    return SFCI_OK;
   }
-  return compact_top<W>(c, ik, ia, n, tau, need_eq, tiny, ok, oa, m);
+  return SFCI_OK;
 }
 
 template <int W>
@@ -898,10 +913,13 @@ int select_sorted(Ctx& c, typename KeyOf<W>::T* keys, double* vals, size_t n, si
       // by magnitude first, so that only what is kept is sorted; ties of the k-th
       // all stay until the keys are in order
       size_t kept = 0;
-      if ((st = select_coop<W>(c, keys, vals, n, 2, k, -1ll, tk, ta, &kept))) return st;
-      SFCI_CUDA(cudaMemcpyAsync(keys, tk, kept * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
-      SFCI_CUDA(cudaMemcpyAsync(vals, ta, kept * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-      n = kept;
+      bool ran = false;
+      if ((st = select_coop<W>(c, keys, vals, n, 2, k, -1ll, tk, ta, &kept, &ran))) return st;
+      if (ran) {
+        SFCI_CUDA(cudaMemcpyAsync(keys, tk, kept * sizeof(KT), cudaMemcpyDeviceToDevice, c.stream));
+        SFCI_CUDA(cudaMemcpyAsync(vals, ta, kept * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+        n = kept;
+      }
     }
   }
   if ((st = radix_sort_pairs<W>(c, keys, vals, n, c.N))) return st;
