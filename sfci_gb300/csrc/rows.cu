@@ -77,6 +77,7 @@ constexpr int MID_BIN = 12;                // MID_MAX = 2^MID_BIN - 1 terms
 constexpr unsigned D1_PIECE = 128;         // entries of one source's doubles a warp takes at a time
 constexpr unsigned PROBE_MAX = 64;         // probes before a table counts as full
 constexpr int NW = 5;                      // accumulator words of a slot
+constexpr int ROW_EL_MAX = 16;             // electrons of a spin (single_elems)
 
 // row packing: terms << 28 | groups two moves away << 11 | groups one move away
 constexpr int RP_D = 11, RP_RAW = 28;
@@ -1257,7 +1258,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
     nb += popc64(kword(k0, w) & 0xaaaaaaaaaaaaaaaaull);
   }
   const int M = c.M, nva = M - na, nvb = M - nb;
-  if (na < 1 || nb < 1 || nva < 1 || nvb < 1 || na > 16 || nb > 16) return SFCI_OK;
+  if (na < 1 || nb < 1 || nva < 1 || nvb < 1 || na > ROW_EL_MAX || nb > ROW_EL_MAX) return SFCI_OK;
   const u64 RA = binom(M, na), RB = binom(M, nb);
   if (RA > ROW_RANKS_MAX || RB > ROW_RANKS_MAX) return SFCI_OK;
   const u64 nsa = (u64)na * nva, nsb = (u64)nb * nvb;
@@ -1513,16 +1514,20 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   const Kern km = d16 ? k_rows_cta<W, 16, MID_THREADS, MID_TB> : k_rows_cta<W, 15, MID_THREADS, MID_TB>;
   const Kern kl = d16 ? k_rows_light<W, 16> : k_rows_light<W, 15>;
   unsigned gb = 0, gm = 0, gl = 0;
-  auto config = [&](Kern k, int threads, size_t sm, unsigned* g) -> int {
+  // (the limit belongs to the kernel, whichever context or thread launches it: always
+  // the most that any system takes, so that no other launch finds it lowered)
+  constexpr unsigned SMAX = ROW_EL_MAX * ((W == 1 ? 32 : 64) - ROW_EL_MAX);
+  auto config = [&](Kern k, int threads, size_t sm, size_t most, unsigned* g) -> int {
     int per = 0;
-    SFCI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    SFCI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     SFCI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, sm));
     if (per < 1) return set_error(SFCI_ERR_CUDA, "row kernel does not fit an SM");
     *g = (unsigned)(c.sm_count * per);
     return SFCI_OK;
   };
-  if ((st = config(kb, Big<W>::threads, smb, &gb)) || (st = config(km, MID_THREADS, smm, &gm)) ||
-      (st = config(kl, LIGHT_WARPS * 32, sml, &gl)))
+  if ((st = config(kb, Big<W>::threads, smb, row_cta_smem<W, Big<W>::tb>(SMAX), &gb)) ||
+      (st = config(km, MID_THREADS, smm, row_cta_smem<W, MID_TB>(SMAX), &gm)) ||
+      (st = config(kl, LIGHT_WARPS * 32, sml, sml, &gl)))
     return st;
   u64 nbig = 0;  // units are ordered by size class, the largest first
   for (int i = MID_BIN; i < BINS; ++i) nbig += bh[i];

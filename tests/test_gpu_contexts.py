@@ -70,3 +70,27 @@ def test_sorts_and_selections_beside_long_products(tmp_path):
         return job
 
     run_together([products, sorts(1), sorts(2)])
+
+
+def test_products_of_systems_of_different_sizes(tmp_path):
+    """The row kernels take 7 words a single excitation of shared memory besides their
+    tables: 45, 115 and 48 of them here.  (A launch that found another thread's
+    smaller limit failed with an invalid value; the window is short, so a run without
+    an error proves little, one with an error all.)"""
+    def job(M, na, n, seed):
+        path = str(tmp_path / ("m%d_IN" % M))
+        fd.rhf_to_in_file(path, M, 2 * na, 3)
+        keys, amps = vector(M, na, na, n, np.random.default_rng(seed))
+
+        def run():
+            c = sg.Context(path, 2 * M, 2 * na, Nd=n)
+            v, out = c.vec_from(keys, amps), c.vec(100000)
+            first = c.SpMVMtply_bucket(v, out, 0.0, 1.0)
+            k, a = out.download()
+            for _ in range(100):
+                assert c.SpMVMtply_bucket(v, out, 0.0, 1.0) == first
+            k1, a1 = out.download()
+            assert np.array_equal(k, k1) and np.array_equal(a, a1)
+        return run
+
+    run_together([job(14, 5, 2500, 1), job(28, 5, 1000, 2), job(16, 4, 2000, 3)])
