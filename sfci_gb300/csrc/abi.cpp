@@ -71,10 +71,12 @@ void scratch_release(Ctx& c, const char* name) {
   c.scratch.erase(it);
 }
 
+bool scratch_is_list(const std::string& name) { return !name.compare(0, 3, "rw_") || !name.compare(0, 3, "pr_"); }
+
 void scratch_release_lists(Ctx& c) {
   cudaStreamSynchronize(c.stream);
   for (auto it = c.scratch.begin(); it != c.scratch.end();) {
-    if (it->first.compare(0, 3, "rw_") && it->first.compare(0, 3, "pr_")) {
+    if (!scratch_is_list(it->first)) {
       ++it;
       continue;
     }

@@ -113,6 +113,7 @@ void scratch_free_all(Ctx& c);
 void scratch_release(Ctx& c, const char* name);
 void scratch_release_plan(Ctx& c);
 void scratch_release_lists(Ctx& c);  // the row product's and the pair search's lists
+bool scratch_is_list(const std::string& name);
 // pinned host words for readbacks
 u64* pinned_words(Ctx& c, size_t n);
 

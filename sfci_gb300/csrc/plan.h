@@ -16,6 +16,19 @@ struct MemPlan {
   int passes = 0;
 };
 
+// Whether the lists that the row product and the pair search keep (`lists` bytes)
+// make way for a plan of T terms of tb bytes.  The plan has the free memory and what
+// it holds already, and wants every term at both levels and through the sort, within
+// the caller's budget (0: none).  Lists of less than 1/64 of that memory stay: the
+// plan would be the same without them, and a solver that alternates the two forms
+// would allocate them anew each time.
+inline bool plan_wants_lists(plan_u64 free, plan_u64 held, plan_u64 lists, plan_u64 T, plan_u64 tb, plan_u64 budget) {
+  const double have = (double)free + (double)held;
+  double want = 3.0 * (double)T * (double)tb + 268435456.0;
+  if (budget) want = std::min(want, (double)budget);
+  return lists > 0 && have * 0.85 < want && (double)lists * 64.0 >= have;
+}
+
 // Generation passes over the level-1 bins for a level-1 capacity c1: consecutive
 // bins are grouped greedily while their terms fit (binoff: nb1 + 1 offsets).
 inline int plan_passes(const std::vector<plan_u64>& binoff, unsigned nb1, plan_u64 c1) {

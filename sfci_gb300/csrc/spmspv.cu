@@ -1648,19 +1648,19 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
   {
     size_t freeb = 0, totb = 0;
     SFCI_CUDA(cudaMemGetInfo(&freeb, &totb));
-    // the row product's and the pair search's lists make way for a plan that cannot
-    // hold every term at both levels beside them
-    if ((double)freeb * 0.85 < 3.0 * (double)T * tb + ((size_t)256 << 20)) {
-      scratch_release_lists(c);
-      SFCI_CUDA(cudaMemGetInfo(&freeb, &totb));
-    }
     // the plan's buffers (replaced in place when they grow): the two term
     // levels and the survivors; the plan also leaves room for the sort scratch
     // the survivors go through (not counted here: whatever it holds stays held)
-    size_t held = 0;
+    size_t held = 0, lists = 0;
     for (const char* nm : {"sp_l1k", "sp_l1a", "sp_l2k", "sp_l2a", "sp_sk", "sp_sa"}) {
       auto it = c.scratch.find(nm);
       if (it != c.scratch.end()) held += it->second.bytes;
+    }
+    for (const auto& kv : c.scratch)
+      if (scratch_is_list(kv.first)) lists += kv.second.bytes;
+    if (plan_wants_lists(freeb, held, lists, T, tb, c.opts.mem_budget)) {
+      scratch_release_lists(c);
+      SFCI_CUDA(cudaMemGetInfo(&freeb, &totb));
     }
     // allocations made after the plan, kept out of it: per leaf the input
     // offsets and cursors, boundaries and overflow lists (24 B), the input
