@@ -43,7 +43,7 @@ void* scratch_get(Ctx& c, const char* name, size_t bytes) {
   void* p = nullptr;
   if (cudaMalloc(&p, want) != cudaSuccess) {
     cudaGetLastError();
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    if (device_malloc(c, &p, bytes) != cudaSuccess) {
       cudaGetLastError();
       set_error(SFCI_ERR_NOMEM, std::string("device allocation of ") + std::to_string(bytes) + " bytes for " + name +
                                     " failed");
@@ -83,6 +83,16 @@ void scratch_release_lists(Ctx& c) {
     if (it->second.p) cudaFree(it->second.p);
     it = c.scratch.erase(it);
   }
+}
+
+cudaError_t device_malloc(Ctx& c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !c.lists_in_use) {
+    cudaGetLastError();
+    scratch_release_lists(c);
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
 }
 
 void scratch_release_plan(Ctx& c) {
@@ -612,8 +622,8 @@ int sfci_vec_create(sfci_ctx* x, uint64_t cap, sfci_vec** out) {
   v->v.cap = cap;
   x->c.live.insert(&v->v);
   size_t n = cap ? cap : 1;
-  cudaError_t e = cudaMalloc(&v->v.keys, n * x->c.W * sizeof(u64));
-  if (e == cudaSuccess) e = cudaMalloc(&v->v.amps, n * sizeof(double));
+  cudaError_t e = device_malloc(x->c, (void**)&v->v.keys, n * x->c.W * sizeof(u64));
+  if (e == cudaSuccess) e = device_malloc(x->c, (void**)&v->v.amps, n * sizeof(double));
   if (e != cudaSuccess) {
     int st = cuda_fail(e, "sfci_vec_create");
     sfci_vec_destroy(v);

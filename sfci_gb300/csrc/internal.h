@@ -53,6 +53,7 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   int sm_count = 0;
   std::map<std::string, Buf> scratch;
+  int lists_in_use = 0;  // ListsInUse objects
   u64 launches = 0;
   cudaEvent_t ev[16] = {};
   // per-phase profiling
@@ -114,6 +115,15 @@ void scratch_release(Ctx& c, const char* name);
 void scratch_release_plan(Ctx& c);
 void scratch_release_lists(Ctx& c);  // the row product's and the pair search's lists
 bool scratch_is_list(const std::string& name);
+// cudaMalloc; where the memory is out, the lists go (none is in use, see below) and
+// it is tried once more.  scratch_get does the same.
+cudaError_t device_malloc(Ctx& c, void** p, size_t bytes);
+// in scope while a row product or a pair search uses its lists
+struct ListsInUse {
+  Ctx& c;
+  explicit ListsInUse(Ctx& c_) : c(c_) { ++c.lists_in_use; }
+  ~ListsInUse() { --c.lists_in_use; }
+};
 // pinned host words for readbacks
 u64* pinned_words(Ctx& c, size_t n);
 

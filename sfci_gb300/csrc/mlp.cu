@@ -1236,7 +1236,7 @@ struct Screen {
 };
 
 static int dev_alloc(Screen& s, void** p, size_t bytes) {
-  if (cudaMalloc(p, bytes ? bytes : 16) != cudaSuccess) {
+  if (device_malloc(*s.ctx, p, bytes ? bytes : 16) != cudaSuccess) {
     cudaGetLastError();
     return set_error(SFCI_ERR_NOMEM, "screen: device allocation failed");
   }

@@ -384,6 +384,7 @@ template <int W, bool ENERGY>
 int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   typedef typename KeyOf<W>::T KT;
   *done = false;
+  const ListsInUse in_use(c);
   int st;
   KT k0;
   if ((st = read_words(c, a.ket.keys, sizeof(KT), &k0))) return st;

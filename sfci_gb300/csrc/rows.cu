@@ -1248,6 +1248,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   typedef typename StrOf<W>::T ST;
   typedef typename KeyOf<W>::T KT;
   *done = false;
+  const ListsInUse in_use(c);
   int st;
   // spin counts of the first source (every other one is checked against them)
   KT k0;

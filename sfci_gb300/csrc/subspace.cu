@@ -316,13 +316,15 @@ namespace {
 
 // device allocations owned by one call
 struct DevArena {
+  Ctx& c;
   std::vector<void*> ps;
+  explicit DevArena(Ctx& c_) : c(c_) {}
   ~DevArena() {
     for (void* p : ps) cudaFree(p);
   }
   void* get(size_t bytes) {
     void* p = nullptr;
-    if (cudaMalloc(&p, bytes ? bytes : 16) != cudaSuccess) {
+    if (device_malloc(c, &p, bytes ? bytes : 16) != cudaSuccess) {
       cudaGetLastError();
       set_error(SFCI_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes for the subspace failed");
       return nullptr;
@@ -537,7 +539,7 @@ int cisd_impl(Ctx& c, const u64* ref_key, int state_idx, int n_evals, double* ev
   if (block_size) *block_size = T;
   if (out.cap < T) return set_error(SFCI_ERR_CAPACITY, "output vector capacity below the CISD block size");
   const int nev = std::max(state_idx + 1, n_evals);
-  DevArena A;
+  DevArena A(c);
   KT* keys = (KT*)A.get(T * sizeof(KT));
   double* tmp = (double*)A.get(T * sizeof(double));
   double* x = (double*)A.get(T * sizeof(double));
@@ -575,7 +577,7 @@ int fci_impl(Ctx& c, int n_evals, double* evals, Vec* ground, double* resid, u64
   const u64 n = nalpha * nbeta;
   if (dim) *dim = n;
   if (ground && ground->cap < n) return set_error(SFCI_ERR_CAPACITY, "ground vector capacity below the FCI dimension");
-  DevArena A;
+  DevArena A(c);
   u64* dbin = (u64*)A.get(binom.size() * sizeof(u64));
   KT* keys = (KT*)A.get(n * sizeof(KT));
   double* tmp = (double*)A.get(n * sizeof(double));
