@@ -54,7 +54,8 @@ typedef struct sfci_opts {
   double coeff_cut;        /* post-merge magnitude cut (0: the default 1e-5, src/main.cpp:196;
                               negative: no cut, every merged determinant is kept) */
   uint64_t bucket_unit;    /* accepted and ignored: sizes come from prefix sums */
-  uint64_t mem_budget;     /* bytes of device scratch the SpMSpV may use (0: 90% of free) */
+  uint64_t mem_budget;     /* bytes of device scratch the SpMSpV, and the searches of sfci_energy and the
+                              linear products' dots, may use (0: 90% of free) */
   int verbose;             /* 1: print the reference's progress lines */
   int reserved[7];
 } sfci_opts;
@@ -89,7 +90,10 @@ int sfci_ctx_profile_read(sfci_ctx* ctx, const char* phase, double* ms, uint64_t
 int sfci_ctx_profile_reset(sfci_ctx* ctx);
 /* Statistics of the last SpMSpV: [0] input dets used, [1] generated terms,
  * [2] merged unique dets, [3] survivors of the cut, [4] output length,
- * [5] passes, [6] leaves, [7] leaves that took the global-memory path. */
+ * [5] passes, [6] leaves (row form: its work units, rows or parts of rows),
+ * [7] leaves that took the global-memory path.  After sfci_energy: [0], [1], and in
+ * [6] the pairs of neighbouring alpha strings its pair search looked at (0: it
+ * generated every term). */
 int sfci_ctx_last_stats(const sfci_ctx* ctx, uint64_t stats[8]);
 
 /* ---- sparse vectors (dynVec, src/all.h:150-625) ------------------------------ */

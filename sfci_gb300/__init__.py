@@ -473,6 +473,8 @@ class Context:
         _check(self.L.sfci_ctx_profile_reset(self.h))
 
     def last_stats(self) -> dict:
+        """Statistics of the last product or energy ("leaves": work units in the row
+        form, pairs of neighbouring alpha strings after an energy by pair search)."""
         a = (C.c_uint64 * 8)()
         _check(self.L.sfci_ctx_last_stats(self.h, a))
         names = ["input_dets", "terms", "unique", "survivors", "out_len", "passes", "leaves", "big_leaves"]

@@ -381,7 +381,7 @@ struct Builder {
 
 // the common part: bras and kets grouped, neighbours listed, k_pairs run
 template <int W, bool ENERGY>
-int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
+int run_pairs(Ctx& c, PairArgs<W>& a, bool* done, u64* links = nullptr) {
   typedef typename KeyOf<W>::T KT;
   *done = false;
   const ListsInUse in_use(c);
@@ -397,6 +397,10 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   if (na < 1 || nb < 1 || nva < 1 || nvb < 1 || na > 16 || nb > 16) return SFCI_OK;
   const u64 RA = binom(M, na);
   if (RA > ROW_RANKS_MAX || a.ket.n >= (1ull << 31) || a.bra.n >= (1ull << 31)) return SFCI_OK;
+  // a device budget holds here too: ranks, then lists, then neighbours
+  u64 need = (RA + 1) * 8 * (ENERGY ? 1 : 2) + a.bra.n * 4 + a.ket.n * 12;
+  auto over = [&](u64 more) { return (need += more) > c.opts.mem_budget && c.opts.mem_budget; };
+  if (over(0)) return SFCI_OK;
   const u64 nsa = (u64)na * nva, nda = (u64)(na * (na - 1) / 2) * (nva * (nva - 1) / 2);
   a.h.N = c.N;
   a.h.M = M;
@@ -443,6 +447,8 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   a.bra.nG = (unsigned)(th[0] >> 32);
   a.ket.nG = (unsigned)(th[1] >> 32);
   if (a.ket.nG * nda >= (1ull << 32)) return SFCI_OK;
+  if (over(((u64)(unsigned)th[0] + (ENERGY ? 0 : (u64)(unsigned)th[1])) * (16 + sizeof(typename StrOf<W>::T))))
+    return SFCI_OK;
   if ((st = b.lists(a.bra, "pr_b", a.RA, na, a.bin, (unsigned)th[0])) || !b.ok) return st;
   if (ENERGY) a.ket = a.bra;
   else if ((st = b.lists(a.ket, "pr_k", a.RA, na, a.bin, (unsigned)th[1])) || !b.ok) return st;
@@ -467,6 +473,7 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   // to 15 times faster.
   if (rb[5] > 4 * a.ket.n * det_terms(na, nva, nb, nvb)) return SFCI_OK;
   const u64 nS = nt & 0xffffffffull, nD = nt >> 32;
+  if (over(nS * 8 + nD * 12)) return SFCI_OK;
   a.nsg = (unsigned*)b.get("pr_nsg", std::max<u64>(1, nS) * 4);
   a.nsx = (unsigned*)b.get("pr_nsx", std::max<u64>(1, nS) * 4);
   a.ndg = (unsigned*)b.get("pr_ndg", std::max<u64>(1, nD) * 4);
@@ -476,6 +483,7 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
   SFCI_LAUNCH(c, (k_pairs<W, ENERGY>), (unsigned)std::max<u64>(1, std::min<u64>((a.ket.n + 7) / 8, b.gmax)), 256, 0, a);
   if ((st = read_words(c, tot + 4, 8, rb))) return st;
   if (rb[0] >> 32) return SFCI_OK;  // out of range: the general sweep reports it
+  if (links) *links = nS + nD;
   *done = true;
   return SFCI_OK;
 }
@@ -484,13 +492,13 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done) {
 
 template <int W>
 int pairs_energy(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 n, double* E, u64* terms,
-                 bool* done) {
+                 u64* links, bool* done) {
   PairArgs<W> a{};
   a.bra.keys = a.ket.keys = keys;
   a.bra.n = a.ket.n = n;
   a.bra.sorted = 1;
   a.amps = a.bamps = amps;
-  int st = run_pairs<W, true>(c, a, done);
+  int st = run_pairs<W, true>(c, a, done, links);
   if (st || !*done) return st;
   u64 s[2];
   if ((st = read_words(c, a.esum, sizeof s, s))) return st;
@@ -515,8 +523,8 @@ int pairs_project(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, 
   return run_pairs<W, false>(c, a, done);
 }
 
-template int pairs_energy<1>(Ctx&, const u64*, const double*, u64, double*, u64*, bool*);
-template int pairs_energy<2>(Ctx&, const K128*, const double*, u64, double*, u64*, bool*);
+template int pairs_energy<1>(Ctx&, const u64*, const double*, u64, double*, u64*, u64*, bool*);
+template int pairs_energy<2>(Ctx&, const K128*, const double*, u64, double*, u64*, u64*, bool*);
 template int pairs_project<1>(Ctx&, const u64*, const double*, u64, double, const u64*, u64, u64*, u64*, bool*);
 template int pairs_project<2>(Ctx&, const K128*, const double*, u64, double, const K128*, u64, u64*, u64*, bool*);
 

@@ -2123,11 +2123,13 @@ int energy_impl(Ctx& c, const Vec& psi, double* E) {
   double* diagE = nullptr;
   if (!c.ninst && psi.len * most_terms(c) >= PAIRS_MIN_TERMS) {
     bool done = false;
-    if ((st = pairs_energy<W>(c, (const KT*)psi.keys, psi.amps, psi.len, E, &T, &done))) return st;
+    u64 links = 0;
+    if ((st = pairs_energy<W>(c, (const KT*)psi.keys, psi.amps, psi.len, E, &T, &links, &done))) return st;
     if (done) {
       for (auto& s : c.stats) s = 0;
       c.stats[0] = psi.len;
       c.stats[1] = T;
+      c.stats[6] = links;
       return SFCI_OK;
     }
   }
