@@ -381,7 +381,7 @@ struct Builder {
 
 // the common part: bras and kets grouped, neighbours listed, k_pairs run
 template <int W, bool ENERGY>
-int run_pairs(Ctx& c, PairArgs<W>& a, bool* done, u64* links = nullptr) {
+int run_pairs(Ctx& c, PairArgs<W>& a, u64 T, u64* links, bool* done) {
   typedef typename KeyOf<W>::T KT;
   *done = false;
   const ListsInUse in_use(c);
@@ -396,6 +396,7 @@ int run_pairs(Ctx& c, PairArgs<W>& a, bool* done, u64* links = nullptr) {
   const int M = c.M, nva = M - na, nvb = M - nb;
   if (na < 1 || nb < 1 || nva < 1 || nvb < 1 || na > 16 || nb > 16) return SFCI_OK;
   const u64 RA = binom(M, na);
+  if (!ENERGY && !pairs_project_pays(T, a.bra.n, RA)) return SFCI_OK;
   if (RA > ROW_RANKS_MAX || a.ket.n >= (1ull << 31) || a.bra.n >= (1ull << 31)) return SFCI_OK;
   // a device budget holds here too: ranks, then lists, then neighbours
   u64 need = (RA + 1) * 8 * (ENERGY ? 1 : 2) + a.bra.n * 4 + a.ket.n * 12;
@@ -498,7 +499,7 @@ int pairs_energy(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.bra.n = a.ket.n = n;
   a.bra.sorted = 1;
   a.amps = a.bamps = amps;
-  int st = run_pairs<W, true>(c, a, done, links);
+  int st = run_pairs<W, true>(c, a, 0, links, done);
   if (st || !*done) return st;
   u64 s[2];
   if ((st = read_words(c, a.esum, sizeof s, s))) return st;
@@ -508,7 +509,7 @@ int pairs_energy(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
 }
 
 template <int W>
-int pairs_project(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 n, double lambda,
+int pairs_project(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u64 n, u64 T, double lambda,
                   const typename KeyOf<W>::T* table, u64 slots, u64* plo, u64* phi, bool* done) {
   PairArgs<W> a{};
   a.ket.keys = keys;
@@ -520,12 +521,12 @@ int pairs_project(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, 
   a.lambda = lambda;
   a.plo = plo;
   a.phi = phi;
-  return run_pairs<W, false>(c, a, done);
+  return run_pairs<W, false>(c, a, T, nullptr, done);
 }
 
 template int pairs_energy<1>(Ctx&, const u64*, const double*, u64, double*, u64*, u64*, bool*);
 template int pairs_energy<2>(Ctx&, const K128*, const double*, u64, double*, u64*, u64*, bool*);
-template int pairs_project<1>(Ctx&, const u64*, const double*, u64, double, const u64*, u64, u64*, u64*, bool*);
-template int pairs_project<2>(Ctx&, const K128*, const double*, u64, double, const K128*, u64, u64*, u64*, bool*);
+template int pairs_project<1>(Ctx&, const u64*, const double*, u64, u64, double, const u64*, u64, u64*, u64*, bool*);
+template int pairs_project<2>(Ctx&, const K128*, const double*, u64, u64, double, const K128*, u64, u64*, u64*, bool*);
 
 }  // namespace sfci

@@ -62,10 +62,10 @@ constexpr int RUN_CAP = 2048;  // class passes: (occupied pair, class block) run
 constexpr double LEAF_TERMS = 1024.0;                 // terms a leaf is sized for (at most, on average)
 
 enum { M_COUNT = 0, M_SCATTER = 1, M_ENERGY = 2, M_PROJECT = 3, M_LABEL = 4 };
-// terms of a full sweep from which the pair search (pairs.cu) is used: its fixed
-// part is some twenty launches, 140 us at 300 sources of 20 spin orbitals (2.6e5
-// terms) against 109 for the sweep, 157 against 159 at 1,000, 173 against 522 at 64
-// of 56 spin orbitals
+// terms of a full sweep from which an energy takes the pair search (pairs.cu; the
+// projections' rule is pairs_project_pays): its fixed part is some twenty launches,
+// 140 us at 300 sources of 20 spin orbitals (2.6e5 terms) against 109 for the sweep,
+// 157 against 159 at 1,000, 176 against 522 at 64 of 56 spin orbitals
 constexpr u64 PAIRS_MIN_TERMS = 1ull << 20;
 constexpr u64 ROWS_MIN_TERMS = 1ull << 20;  // below it rows_product never pays (rows.cu has the rule)
 constexpr int PROJ_MAX = 64;  // vectors of one projection sweep
@@ -2244,8 +2244,10 @@ int project_impl(Ctx& c, const Vec& src, double lambda, const Vec* const* basis,
   }
   int st;
   bool done = false;
-  if (!c.ninst && src.len * most_terms(c) >= PAIRS_MIN_TERMS) {
-    if ((st = pairs_project<W>(c, (const KT*)src.keys, src.amps, src.len, lambda, tk, tsz, plo, phi, &done))) return st;
+  const u64 most = src.len * most_terms(c);
+  if (!c.ninst && pairs_project_pays(most, tsz, 1)) {
+    if ((st = pairs_project<W>(c, (const KT*)src.keys, src.amps, src.len, most, lambda, tk, tsz, plo, phi, &done)))
+      return st;
     if (!done) SFCI_CUDA(cudaMemsetAsync(acc, 0, (2 * tsz + 1) * sizeof(u64), c.stream));
   }
   if (!done) {

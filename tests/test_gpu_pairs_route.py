@@ -76,3 +76,28 @@ def test_a_full_space_takes_the_sweep(tmp_path):
     v, out = c.vec_from(keys, amps), c.vec(len(keys))
     d = c.SpMVMtply_bucket(v, out, 0.0, 1.0)
     assert abs(c.calc_energy(v) - d) < 1e-13 and c.last_stats()["leaves"] == 0
+
+
+@pytest.mark.parametrize("M,n,B,search", [(28, 64, 20000, False), (28, 1000, 1000, True), (34, 300, 20000, False)])
+def test_a_short_vector_on_a_long_basis_takes_the_sweep(M, n, B, search, tmp_path):
+    """1.2e6 terms against 65,536 slots, 1.8e7 against 2,048, 8.8e6 against 65,536 with
+    280,000 strings of a spin.  The dot with the basis whole and in two halves is the
+    same sum but for its additions: at most 30 roundings in a row (a thread's few and
+    two trees of 256), of partial sums below |v| |H| = 100, 3.4e-13."""
+    path = str(tmp_path / "sys_IN")
+    fd.rhf_to_in_file(path, M, 10, 3)
+    rng = np.random.default_rng(41)
+    keys, amps = vector(M, 5, 5, n, rng)
+    kb, ab = vector(M, 5, 5, B, rng)
+    c = sg.Context(path, 2 * M, 10, Nd=n, mem_budget=64 << 30)
+    v, out, b = c.vec_from(keys, amps), c.vec(400000), c.vec_from(kb, ab)
+    made = []
+    for f in (lambda: c.SpMVMtply_bucket(v, out, 0.5, 1.0), lambda: c.spmspvm_bucket_linear(v, out, 0.5, [b])):
+        f()
+        k = c.launches()
+        f()
+        made.append(c.launches() - k)
+    assert (made[1] - made[0] > 24) == search
+    whole = c.spmspvm_bucket_linear(v, out, 0.5, [b])
+    parts = c.spmspvm_bucket_linear(v, out, 0.5, [c.vec_from(kb[::2], ab[::2]), c.vec_from(kb[1::2], ab[1::2])])
+    assert abs(whole[0] - parts.sum()) <= 1e-12
