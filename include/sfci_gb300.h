@@ -256,8 +256,10 @@ int sfci_batch_lanczos(sfci_ctx* ctx, sfci_vec* const* v, int n, int Nl, int res
                        double* final_e);
 /* Product plan tunables {level-1 bits 4-9, partition digit bits 6-9, distinct keys
  * per leaf 16-120, generation CTAs per SM 1-2}: they change speed, never results
- * (the merge is exact).  sfci_autotune times candidate plans on the product of
- * `in` (into `out`), checks that they agree, and keeps the fastest. */
+ * (the merge is exact).  They shape the partitioned products (batched, screened,
+ * within a device budget, with a sum of squares, and those the row form declines).
+ * sfci_autotune times candidate plans on the partitioned product of `in` (into
+ * `out`), checks that they agree, and keeps the fastest. */
 int sfci_ctx_set_tuning(sfci_ctx* ctx, const int* tuning4);
 /* Generation passes of a product whose terms exceed the device budget: by ranges
  * of the targets' alpha class (mode 0: when three or more passes are needed; 1:

@@ -457,6 +457,13 @@ int sfci_autotune(sfci_ctx* x, const sfci_vec* in, sfci_vec* out, int* best4, do
   static const int cand[][4] = {{9, 9, 120, 2}, {9, 8, 120, 2}, {8, 9, 120, 2}, {9, 9, 80, 2},
                                 {9, 9, 60, 2},  {9, 9, 120, 1}, {7, 8, 120, 2}, {9, 8, 80, 2}};
   const int save[4] = {c.tune_l1_bits, c.tune_digit_bits, c.tune_leaf_uniq, c.tune_gen_ctas};
+  // the tunables shape the partitioned pipeline: it is what the candidates time, also
+  // where the row form takes this context's plain products
+  struct Tuning {
+    Ctx& c;
+    explicit Tuning(Ctx& c_) : c(c_) { c.tuning = true; }
+    ~Tuning() { c.tuning = false; }
+  } tuning(c);
   double best = 1e300;
   int bi = 0;
   uint64_t ref_len = 0;

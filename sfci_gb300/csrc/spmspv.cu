@@ -1572,10 +1572,10 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
   }
   // Row-driven form: whole products on one plain Hamiltonian.  The partitioned
   // pipeline below takes the rest (sums of squares, screens, batches), the plans a
-  // caller asked for by a device budget or by class passes, and what
-  // rows_product declines.
+  // caller asked for by a device budget or by class passes, the plans that the
+  // autotuner times, and what rows_product declines.
   if (!(ex && ex->sumsq) && !(c.screen && ng == ns) && !c.ninst && !c.opts.mem_budget && c.tune_class_passes <= 0 &&
-      ns * conn >= ROWS_MIN_TERMS) {
+      !c.tuning && ns * conn >= ROWS_MIN_TERMS) {
     RowsResult<W> rr;
     bool done = false;
     phase_end(c, tok);
