@@ -90,7 +90,7 @@ int sfci_ctx_profile_read(sfci_ctx* ctx, const char* phase, double* ms, uint64_t
 int sfci_ctx_profile_reset(sfci_ctx* ctx);
 /* Statistics of the last SpMSpV: [0] input dets used, [1] generated terms,
  * [2] merged unique dets, [3] survivors of the cut, [4] output length,
- * [5] passes, [6] leaves (row form: its work units, rows or parts of rows),
+ * [5] passes (row form: fillings of its survivor buffer), [6] leaves (row form: its work units, rows or parts of rows),
  * [7] leaves that took the global-memory path.  After sfci_energy: [0], [1], and in
  * [6] the pairs of neighbouring alpha strings its pair search looked at (0: it
  * generated every term). */
@@ -267,6 +267,11 @@ int sfci_ctx_set_tuning(sfci_ctx* ctx, const int* tuning4);
  * its own terms, or by hash bins, each pass regenerating every term.  Results
  * never depend on the mode. */
 int sfci_ctx_set_class_passes(sfci_ctx* ctx, int mode);
+/* Survivors of the cut that a row-form product holds beyond its output's capacity
+ * before it keeps the largest of them and goes on (0, the default: 1/64 of the
+ * device memory, at least 2^24).  A smaller margin takes less memory and, where more
+ * survive, more rounds; the results are the same. */
+int sfci_ctx_set_row_margin(sfci_ctx* ctx, uint64_t entries);
 /* Key sort and magnitude selection as one launch each, whose blocks wait for one
  * another (1, the default), or as a chain of launches without such a wait (0), which
  * is also what runs where the GPU cannot hold the one launch's grid.  The results

@@ -102,6 +102,7 @@ def _sigs(L):
     L.sfci_batch_lanczos.argtypes = [_vp, C.POINTER(_vp), C.c_int, C.c_int, C.c_int, _vp, _vp]
     L.sfci_ctx_set_tuning.argtypes = [_vp, _vp]
     L.sfci_ctx_set_class_passes.argtypes = [_vp, C.c_int]
+    L.sfci_ctx_set_row_margin.argtypes = [_vp, C.c_uint64]
     L.sfci_ctx_set_grid_barrier.argtypes = [_vp, C.c_int]
     L.sfci_ctx_get_tuning.argtypes = [_vp, _vp]
     L.sfci_autotune.argtypes = [_vp, _vp, _vp, _vp, C.POINTER(C.c_double)]
@@ -288,6 +289,10 @@ class Context:
     def set_class_passes(self, mode: int):
         """Generation passes by target alpha class: 0 when needed, 1 always, -1 never."""
         _check(self.L.sfci_ctx_set_class_passes(self.h, int(mode)))
+
+    def set_row_margin(self, entries: int):
+        """Survivors a row-form product holds beyond its output's capacity (0: by the device memory)."""
+        _check(self.L.sfci_ctx_set_row_margin(self.h, int(entries)))
 
     def set_grid_barrier(self, on: bool):
         """Sort and select in one launch each, with a grid barrier (the default), or in several without."""

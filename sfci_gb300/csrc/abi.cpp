@@ -433,6 +433,12 @@ int sfci_ctx_set_class_passes(sfci_ctx* x, int mode) {
   return SFCI_OK;
 }
 
+int sfci_ctx_set_row_margin(sfci_ctx* x, uint64_t entries) {
+  if (!x || entries > (1ull << 40)) return set_error(SFCI_ERR_ARG, "row margin: a context and at most 2^40 entries");
+  x->c.tune_row_margin = entries;
+  return SFCI_OK;
+}
+
 int sfci_ctx_set_grid_barrier(sfci_ctx* x, int on) {
   if (!x) return set_error(SFCI_ERR_ARG, "null context");
   x->c.grid_barrier = on != 0;

@@ -85,6 +85,7 @@ struct Ctx {
   int tune_digit_bits = 9;    // most bits per partition level
   int tune_leaf_uniq = 120;   // distinct keys a leaf is sized for
   int tune_gen_ctas = 2;      // generation CTAs per SM
+  uint64_t tune_row_margin = 0;  // survivors the row form holds beyond the output's capacity (0: by memory)
   bool tuning = false;        // the autotuner is timing plans: every product takes one
   int tune_class_passes = 0;  // generation passes by target alpha class: 0 when needed, 1 always, -1 never
   // learned excitation screen applied by the products (nullptr: plain products)

@@ -1297,7 +1297,8 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   for (auto& kv : c.scratch)
     if (kv.first.compare(0, 3, "rw_") == 0) mine += kv.second.bytes;
   const size_t avail = (size_t)((freeb + held + mine) * 0.9);
-  const u64 margin = std::min<u64>(T, std::max<u64>(1ull << 24, avail / 64 / (sizeof(KT) + 8)));
+  const u64 margin =
+      std::min<u64>(T, c.tune_row_margin ? c.tune_row_margin : std::max<u64>(1ull << 24, avail / 64 / (sizeof(KT) + 8)));
   const u64 slack = (u64)c.sm_count * 10240;  // an SM's shared memory holds fewer table slots than that
   const u64 SC = std::min<u64>(cap, T) + margin + slack;
   size_t need = (nx ? RA * 8 + nx * (sizeof(ST) + 12) : 0) + RA * 40 + RB * 8 + ns * (nsb * (sizeof(ST) + 4 + 6) + 64) + SC * 2 * (sizeof(KT) + 8) + ((size_t)64 << 20);
@@ -1588,6 +1589,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
     size_t m = 0;
     if ((st = select_sorted<W>(c, a.sk, a.sa, nsurv, cap, &m))) return st;
     out->pruned = true;
+    ++out->rounds;
     const u64 m64 = m;
     SFCI_CUDA(cudaMemcpyAsync(scount, &m64, 8, cudaMemcpyHostToDevice, c.stream));
     SFCI_CUDA(cudaMemsetAsync(a.ucur, 0, 4, c.stream));

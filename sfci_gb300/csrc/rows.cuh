@@ -16,6 +16,7 @@ struct RowsResult {
   u64 terms = 0;     // generated terms
   u64 dexact[2] = {0, 0};  // <v|Hv>, exact 128-bit fixed point
   u64 units = 0;     // work units
+  u64 rounds = 1;       // fillings of the survivor buffer
   bool pruned = false;  // survivors were cut to the output capacity on the way
 };
 

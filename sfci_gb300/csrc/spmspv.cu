@@ -1584,7 +1584,7 @@ int spmspv_impl(Ctx& c, const Vec& in, Vec& out, double lambda, double coeff, do
       c.stats[1] = rr.terms;
       c.stats[2] = rr.uniq;
       c.stats[3] = rr.nsurv;
-      c.stats[5] = 1;
+      c.stats[5] = rr.rounds;
       c.stats[6] = rr.units;
       c.last_pruned = rr.pruned;
       if (rr.uniq) c.dup_est = (double)rr.terms / (double)rr.uniq;
