@@ -465,9 +465,9 @@ __global__ void __launch_bounds__(ROW_T, 1) k_mlp_fwd(FwdArgs a) {
           o.w = pack_bf16(g2[8 * q + 6], g2[8 * q + 7]);
           *reinterpret_cast<uint4*>(sA + umma::tile_offset(row, 32 * k + 8 * q, HID)) = o;
         }
-        const float cb = lane_column_sum(g2), cw = lane_column_sum(gw);
-        atomicAdd(sg_b2 + 32 * k + lane, cb);
-        atomicAdd(sg_w3 + 32 * k + lane, cw);
+        const float sum2 = lane_column_sum(g2), sum3 = lane_column_sum(gw);
+        atomicAdd(sg_b2 + 32 * k + lane, sum2);
+        atomicAdd(sg_w3 + 32 * k + lane, sum3);
       }
       if (part == 0) {
         const float d3s = warp_sum(d3);
@@ -1032,8 +1032,8 @@ __global__ void __launch_bounds__(ROW_T, 1) k_mlp_bwd(BwdArgs a) {
         o.w = pack_bf16(z[8 * q + 6], z[8 * q + 7]);
         *reinterpret_cast<uint4*>(sA + umma::tile_offset(row, 32 * k + 8 * q, HID)) = o;
       }
-      const float cb = lane_column_sum(z);
-      atomicAdd(sg_b1 + 32 * k + lane, cb);
+      const float sum1 = lane_column_sum(z);
+      atomicAdd(sg_b1 + 32 * k + lane, sum1);
     }
     __syncthreads();
     export_transposed(sA, a.D1T + (size_t)t * T256_BYTES);

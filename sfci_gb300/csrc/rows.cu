@@ -1306,6 +1306,12 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   if (need > freeb + mine) scratch_release_plan(c);
   if (!row_tables(c, a.h)) return SFCI_OK;
   int tok = phase_begin(c, PH_COUNT);
+  // the phase open at a return is closed with it (one already closed is left alone)
+  struct ClosePhase {
+    Ctx& c;
+    const int& tok;
+    ~ClosePhase() { phase_end(c, tok); }
+  } close_phase{c, tok};
   bool ok = true;
   auto get = [&](const char* nm, size_t bytes) -> void* {
     void* p = scratch_get(c, nm, bytes);
@@ -1362,10 +1368,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   SFCI_CUDA(cudaMemcpyAsync(tot + 2, a.flag, 16, cudaMemcpyDeviceToDevice, c.stream));
   u64 th[8];
   if ((st = read_words(c, tot, 4 * 8, th))) return st;
-  if ((unsigned)th[2]) {
-    phase_end(c, tok);
-    return SFCI_OK;
-  }
+  if ((unsigned)th[2]) return SFCI_OK;
   a.nG = (unsigned)(th[0] >> 32);
   a.nB = (unsigned)th[1];
   // pairs of groups and the rows they reach: 12 B each (and the same for the
@@ -1376,10 +1379,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   while (db < 10 && (4ull << db) < ndb) ++db;
   a.db = db;
   need += nSent * 8 + nDent * 12 + a.nB * (nsb * (sizeof(ST) + 2) + ndb * (sizeof(ST) + 8) + ((2ull << db) + 4));
-  if (need > avail || nSent >= (1ull << 31) || nDent >= (1ull << 31) || a.nB * ndb >= (1ull << 32)) {
-    phase_end(c, tok);
-    return SFCI_OK;
-  }
+  if (need > avail || nSent >= (1ull << 31) || nDent >= (1ull << 31) || a.nB * ndb >= (1ull << 32)) return SFCI_OK;
   if (need > freeb + mine) scratch_release_plan(c);
   const u64 nb0max = 2 * ns + a.nG, nb1max = ns * nsb + a.nG;  // at most n buckets for n entries
   a.gstr = (ST*)get("rw_gstr", a.nG * sizeof(ST));
@@ -1422,10 +1422,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
     a.xH = (ST*)get("rw_xH", nx * sizeof(ST));
     a.xv = (double*)get("rw_xv", nx * 8);
   }
-  if (!ok) {
-    phase_end(c, tok);
-    return SFCI_OK;
-  }
+  if (!ok) return SFCI_OK;
   SFCI_CUDA(cudaMemsetAsync(a.rpack, 0, RA * 8, c.stream));
   if (nx) {
     SFCI_CUDA(cudaMemsetAsync(a.xc, 0, RA * 4, c.stream));
@@ -1472,10 +1469,8 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   u64 nunits = 0;
   for (int i = 0; i < BINS; ++i) nunits += bh[i];
   a.nlight = bh[BINS];
-  if ((unsigned)th[1] || maxg >= (1u << 19) || nb0 > nb0max || nb1 > nb1max || nunits + a.nlight >= (1ull << 31)) {
-    phase_end(c, tok);
+  if ((unsigned)th[1] || maxg >= (1u << 19) || nb0 > nb0max || nb1 > nb1max || nunits + a.nlight >= (1ull << 31))
     return SFCI_OK;
-  }
   const u64 nall = nunits + a.nlight;
   a.units = (uint4*)get("rw_units", std::max<u64>(1, nunits) * sizeof(uint4));
   a.light = (unsigned*)get("rw_light", std::max<u64>(1, a.nlight) * 4);
@@ -1484,10 +1479,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   a.sk = (KT*)get("sp_sk", SC * sizeof(KT));
   a.sa = (double*)get("sp_sa", SC * sizeof(double));
   u64* scount = (u64*)get("rw_scount", 4 * 8);
-  if (!ok) {
-    phase_end(c, tok);
-    return SFCI_OK;
-  }
+  if (!ok) return SFCI_OK;
   a.scount = scount;
   a.dexact = scount + 2;
   a.soft = SC - slack;
@@ -1571,10 +1563,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
     SFCI_CUDA(cudaMemcpyAsync(rb + 6, a.nredo, 4, cudaMemcpyDeviceToDevice, c.stream));
     u64 buf[7];
     if ((st = read_words(c, rb, sizeof buf, buf))) return st;
-    if ((unsigned)(buf[4] >> 32)) {  // a term above 2^max_exp
-      phase_end(c, tok);
-      return SFCI_OK;
-    }
+    if ((unsigned)(buf[4] >> 32)) return SFCI_OK;  // a term above 2^max_exp
     nsurv = buf[0];
     out->uniq = buf[1];
     out->dexact[0] = buf[2];
