@@ -316,21 +316,21 @@ SFCI_HD double fx_to_double(u64 lo, u64 hi) {
   return bits_dbl((neg << 63) | ((u64)(top - FX_FRAC + 1023) << 52) | (mant & 0xfffffffffffffull));
 }
 
-// x * 2^(FX_FRAC + up) rounded to the nearest integer (ties to even), as a 128-bit
-// two's-complement (h:l); sets *bad for |x| * 2^up >= 2^62 or not finite (then 0).
+// x * 2^FX_FRAC rounded to the nearest integer (ties to even), as a 128-bit
+// two's-complement (h:l); sets *bad for |x| >= 2^62 or not finite (then 0).
 // The wide form for sums with more terms than the split accumulators take.
-SFCI_HD void fx128_of(double x, u64& l, u64& h, unsigned& bad, int up = 0) {
+SFCI_HD void fx128_of(double x, u64& l, u64& h, unsigned& bad) {
   const u64 b = dbl_bits(x);
-  const int e0 = (int)((b >> 52) & 0x7ff), e = e0 + up;
+  const int e = (int)((b >> 52) & 0x7ff);
   const u64 m = (b & 0xfffffffffffffull) | (1ull << 52);
   const int s = e - (1075 - FX_FRAC);  // F = m * 2^s
   l = 0;
   h = 0;
-  if (e >= 1023 + 62 || e0 == 0x7ff) {
+  if (e >= 1023 + 62) {
     bad = 1u;
     return;
   }
-  if (e0 == 0 || s < -53) return;
+  if (e == 0 || s < -53) return;
   if (s < 0) {
     l = shr_round(m, -s);
   } else if (s < 64) {

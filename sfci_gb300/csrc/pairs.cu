@@ -72,7 +72,8 @@ struct PairArgs {
   double lambda;
   const double* bamps;  // ENERGY: of the bras
   u64* esum;            // ENERGY: exact 128-bit sum of the products times 4^up
-  int up;               // ENERGY: power of two that brings the largest amplitude into [1, 2)
+  int up;               // ENERGY: power of two that brings the largest amplitude into [1, 2),
+  double up2;           // and 4^up, by which the kets are multiplied
   u64 *plo, *phi;       // PROJECT: exact sums by bra index (split form)
 };
 
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(256) k_pairs(PairArgs<W> a) {
     amp = signed_by(par ^ (x >> 31), amp);
     if (ENERGY) {
       u64 l, h;
-      fx128_of(amp * a.bamps[x & 0x7fffffffu], l, h, bad, a.up);
+      fx128_of(amp * a.bamps[x & 0x7fffffffu], l, h, bad);
       slo += l;
       shi += h + (slo < l ? 1ull : 0ull);
     } else {
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(256) k_pairs(PairArgs<W> a) {
   for (u64 p = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < k.n; p += nw) {
     const unsigned g = k.pg[p], x = k.px[p];
     const ST A = k.gstr[g], H = k.pH[p], B = hs_inv(H);
-    const double c0 = ENERGY ? scalbn(a.amps[x & 0x7fffffffu], a.up) : a.amps[x & 0x7fffffffu];
+    const double c0 = ENERGY ? a.up2 * a.amps[x & 0x7fffffffu] : a.amps[x & 0x7fffffffu];
     const double c = signed_by(x >> 31, c0);
     const u64 o0 = a.noff[g], o1 = a.noff[g + 1];
     // groups one move away
@@ -441,10 +442,11 @@ int run_pairs(Ctx& c, PairArgs<W>& a, u64 T, u64* links, bool* done) {
   u64 th[5], rb[6];
   if ((st = read_words(c, tot, sizeof th, th))) return st;
   if ((unsigned)th[4]) return SFCI_OK;
-  // (subnormal largest amplitudes: the energy is zero; not finite: no scaling, and
-  // the sum reports it)
-  const int emax = (int)(th[3] >> 52);
-  if (ENERGY && emax < 0x7ff) a.up = std::min(1022, 1023 - emax);
+  if (ENERGY) {
+    a.up = 1023 - (int)(th[3] >> 52);
+    if (th[3] && std::abs(a.up) > 500) return SFCI_OK;  // (infinities and NaNs too) left to the sweep
+    a.up2 = std::ldexp(1.0, th[3] ? 2 * a.up : 0);
+  }
   a.bra.nG = (unsigned)(th[0] >> 32);
   a.ket.nG = (unsigned)(th[1] >> 32);
   if (a.ket.nG * nda >= (1ull << 32)) return SFCI_OK;
@@ -503,7 +505,7 @@ int pairs_energy(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   if (st || !*done) return st;
   u64 s[2];
   if ((st = read_words(c, a.esum, sizeof s, s))) return st;
-  *E = std::ldexp(fx_to_double(s[0], s[1]), -2 * a.up);
+  *E = fx_to_double(s[0], s[1]) / a.up2;
   *terms = n * det_terms(a.na, a.nva, a.nb, c.M - a.nb);
   return SFCI_OK;
 }

@@ -862,8 +862,8 @@ __global__ void __launch_bounds__(NT, (W == 1 ? 1024 : 768) / NT) k_rows_cta(Row
   for (;;) {
     if (tid == 0) {
       // (no more units once a term was too large: the product is then declined)
-      const unsigned u = *(volatile unsigned*)(a.flag + 1) ? ~0u : atomicAdd(a.ucur, 1u);
-      s_unit = u < a.nunits ? a.units[u] : make_uint4(0u, 1u, 0u, 0u);
+      const unsigned stop = *(volatile unsigned*)(a.flag + 1), u = atomicAdd(a.ucur, 1u);
+      s_unit = u < a.nunits && !stop ? a.units[u] : make_uint4(0u, 1u, 0u, 0u);
     }
     __syncthreads();
     const uint4 un = s_unit;
@@ -1356,10 +1356,16 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   const unsigned gmax = (unsigned)c.sm_count * 8;
   auto grid_of = [&](u64 n, unsigned per) { return (unsigned)std::max<u64>(1, std::min<u64>((n + per - 1) / per, gmax)); };
   SFCI_LAUNCH(c, k_rows_split<W>, grid_of(ns, 256), 256, 0, a);
-  SFCI_LAUNCH(c, k_rows_diag<W>, (unsigned)std::max<u64>(1, std::min<u64>((ns + 7) / 8, gmax * 2)), 256, 0, a, diagE);
+  // the diagonal elements need nothing but the sources: beside the rank tables' scans
+  SideWork side(c);
+  if ((st = side.begin())) return st;
+  k_rows_diag<W><<<(unsigned)std::max<u64>(1, std::min<u64>((ns + 7) / 8, gmax * 2)), 256, 0, c.side>>>(a, diagE);
+  c.launches++;
+  SFCI_CUDA(cudaGetLastError());
   SFCI_LAUNCH(c, k_rows_mark, grid_of(RA, 256), 256, 0, a.arank, a.RA);
   if ((st = scan_excl(c, a.arank, a.arank, RA))) return st;
   if ((st = scan_excl_u32(c, a.brank, a.brank, RB))) return st;
+  side.join();
   // the counts the host sizes the rest from
   u64* tot = (u64*)get("rw_tot", 8 * 8);
   if (!ok) return SFCI_OK;
@@ -1433,7 +1439,6 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   SFCI_CUDA(cudaMemsetAsync(a.rcur, 0, RA * 8, c.stream));
   SFCI_LAUNCH(c, k_rows_groups<W>, grid_of(std::max(RA, RB), 256), 256, 0, a);
   // the beta strings' doubles need nothing but the strings: beside the lists below
-  SideWork side(c);
   if (ndb) {
     if ((st = side.begin())) return st;
     k_rows_bdoubles<W><<<grid_of(a.nB, 1), 256, sizeof(uint32_t) << db, c.side>>>(a);
