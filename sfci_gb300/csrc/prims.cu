@@ -962,8 +962,7 @@ __global__ void k_sumsq_part(const double* __restrict__ a, size_t n, double* __r
 }
 
 // Partial sums added by one CTA.  A dependent FP64 addition takes about 150 cycles
-// on this GPU, so a serial chain over 512 partials cost 40 us (683 of a dot: 50);
-// the tree takes 3.  It adds in twice the working precision, so no rounding is
+// on this GPU, so a serial chain over 512 partials cost 40 us; the tree takes 3.  It adds in twice the working precision, so no rounding is
 // added to the partial sums' but the last.
 constexpr int SUM_THREADS = 256;
 
@@ -980,7 +979,7 @@ int sum_parts(Ctx& c, const double* p, u64 n, double* out) {
   return SFCI_OK;
 }
 
-// The same with the squares (each rounded once) added in twice the working
+// The same with the squares, rounding errors and all, added in twice the working
 // precision, for vectors short enough that the seven FP64 operations an entry (an
 // SM issues two a cycle) stay below the launch and readback: 5 us at 400,000
 // entries.  The sum is then that of the squares, rounded once but for rare cases.
@@ -991,7 +990,7 @@ __global__ void __launch_bounds__(256) k_sumsq_part2(const double* __restrict__ 
   __shared__ double sh[512];
   double hi = 0.0, lo = 0.0;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    two_sum(hi, lo, a[i] * a[i], 0.0);
+    two_prod_sum(hi, lo, a[i], a[i]);
   const double t = block_sum2<256>(hi, lo, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = t;
 }

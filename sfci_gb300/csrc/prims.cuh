@@ -51,27 +51,52 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// (hi, lo) += (bh, bl), exact up to the rounding of the error terms (Knuth's two-sum)
+// (hi, lo) += (bh, bl), exact up to the rounding of the error terms (Dekker's sum of
+// two numbers with the larger one first, which an integer comparison finds: three FP64
+// additions in a row where Knuth's two-sum has six, of which an SM takes two a cycle)
 __device__ __forceinline__ void two_sum(double& hi, double& lo, double bh, double bl) {
-  const double s = hi + bh, t = s - hi, e = (hi - (s - t)) + (bh - t);
+  const bool sw = abs_bits(hi) < abs_bits(bh);
+  const double x = sw ? bh : hi, y = sw ? hi : bh, s = x + y, e = y - (s - x);
   hi = s;
   lo += bl + e;
 }
 // a compensated sum as a double (infinities and NaNs: their error terms are NaN)
 __device__ __forceinline__ double two_value(double hi, double lo) { return isfinite(hi) ? hi + lo : hi; }
-// sum of every thread's (hi, lo); valid in thread 0.  Warp 0 adds NT / 32 pairs a
-// lane before its tree: a tree over all threads would issue three times the FP64
-// additions, of which an SM takes two a cycle.
+// (hi, lo) += a * b, the product's own rounding error included (Knuth's two-sum with
+// fused products: one FP64 operation on hi's path from one call to the next)
+__device__ __forceinline__ void two_prod_sum(double& hi, double& lo, double a, double b) {
+  const double s = __fma_rn(a, b, hi), t = s - hi;
+  lo += (hi - (s - t)) + __fma_rn(a, b, -t);
+  hi = s;
+}
+// sum of every thread's (hi, lo); valid in thread 0.  Four warps add NT / 128 pairs a
+// lane, then each its lanes, then the first their four sums: eight dependent additions
+// for 256 threads.  (A tree over all threads would issue more FP64 additions than hide
+// behind one another; one warp for the whole tree had twelve in a row.)
 template <int NT>
 __device__ __forceinline__ double block_sum2(double hi, double lo, double* sh /* 2 * NT */) {
   sh[threadIdx.x] = hi;
   sh[NT + threadIdx.x] = lo;
   __syncthreads();
-  if (threadIdx.x < 32) {
+  if (threadIdx.x < 128) {
 #pragma unroll
-    for (int q = 1; q < NT / 32; ++q) two_sum(hi, lo, sh[q * 32 + threadIdx.x], sh[NT + q * 32 + threadIdx.x]);
+    for (int q = 1; q < NT / 128; ++q) two_sum(hi, lo, sh[q * 128 + threadIdx.x], sh[NT + q * 128 + threadIdx.x]);
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
+      const double bh = __shfl_xor_sync(0xffffffffu, hi, o), bl = __shfl_xor_sync(0xffffffffu, lo, o);
+      two_sum(hi, lo, bh, bl);
+    }
+    if ((threadIdx.x & 31) == 0) {  // (its own slots, which only it has read)
+      sh[threadIdx.x] = hi;
+      sh[NT + threadIdx.x] = lo;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    hi = sh[32 * (threadIdx.x & 3)];
+    lo = sh[NT + 32 * (threadIdx.x & 3)];
+#pragma unroll
+    for (int o = 2; o; o >>= 1) {
       const double bh = __shfl_xor_sync(0xffffffffu, hi, o), bl = __shfl_xor_sync(0xffffffffu, lo, o);
       two_sum(hi, lo, bh, bl);
     }

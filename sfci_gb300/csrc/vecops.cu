@@ -58,28 +58,77 @@ __global__ void k_merge(const KT* __restrict__ A, const double* __restrict__ Aa,
 }
 
 // dot over common keys (keys unique within each vector); the products of matches,
-// a few a thread, are summed in twice the working precision
-template <class KT>
-__global__ void k_dot(const KT* __restrict__ A, const double* __restrict__ Aa, u64 na, const KT* __restrict__ B,
-                      const double* __restrict__ Ba, u64 nb, double* __restrict__ part) {
+// a few a thread, are summed in twice the working precision, and the last block to
+// finish adds the blocks' sums.  Bound by latency and by the FP64 additions, of which
+// a warp makes an entry's whenever one lane matches: a thread's matches wait until its
+// entries are through (at most every second one matches where keys do not repeat), and
+// short vectors take fewer entries a thread, so that every SM has some.  Whole calls,
+// us, with eight entries a thread, a sum per match and a second launch for the blocks'
+// sums, and now: 1,000 and 500 entries 29.5 and 24.5, 100,000 and 50,000 38 and 26.5,
+// 1,000,000 and 500,000 62.5 and 54.6, two-word keys 38 and 24.5, 38 and 28.4, 75.7 and 75.7.
+template <class KT, int ITEMS>
+__global__ void __launch_bounds__(MP_THREADS) k_dot(const KT* __restrict__ A, const double* __restrict__ Aa, u64 na,
+                                                    const KT* __restrict__ B, const double* __restrict__ Ba, u64 nb,
+                                                    double* part, unsigned* ticket, double* out) {
   __shared__ double sh[2 * MP_THREADS];
+  __shared__ bool s_last;
   const u64 n = na + nb;
-  u64 d = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * MP_ITEMS;
-  double acc = 0.0, low = 0.0;
+  u64 d = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * ITEMS;
+  // matches that wait, the latest first (not with eight entries of two-word keys: the
+  // registers would cost more blocks an SM than the additions saved)
+  constexpr int H = sizeof(KT) > 8 && ITEMS > 4 ? 1 : ITEMS / 2;
+  double acc = 0.0, low = 0.0, pa[H], pb[H];
+  int m = 0;
   if (d < n) {
     u64 i = merge_path(A, na, B, nb, d), j = d - i;
-    for (int t = 0; t < MP_ITEMS && d + t < n; ++t) {
+    for (int t = 0; t < ITEMS && d + t < n; ++t) {
       bool takeA = (j >= nb) || (i < na && !key_lt(B[j], A[i]));
       if (takeA) {
         ++i;
       } else {
-        if (i > 0 && key_eq(A[i - 1], B[j])) two_sum(acc, low, Aa[i - 1] * Ba[j], 0.0);
+        if (i > 0 && key_eq(A[i - 1], B[j])) {
+          if (m == H) two_prod_sum(acc, low, pa[H - 1], pb[H - 1]);
+          else ++m;
+#pragma unroll
+          for (int q = H - 1; q > 0; --q) {
+            pa[q] = pa[q - 1];
+            pb[q] = pb[q - 1];
+          }
+          pa[0] = Aa[i - 1];
+          pb[0] = Ba[j];
+        }
         ++j;
       }
     }
   }
-  const double t = block_sum2<MP_THREADS>(acc, low, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
+  __syncwarp();
+#pragma unroll
+  for (int q = H - 1; q >= 0; --q)
+    if (q < m) two_prod_sum(acc, low, pa[q], pb[q]);
+  double t = block_sum2<MP_THREADS>(acc, low, sh);
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) *out = t;
+    return;
+  }
+  if (!ticket) {
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    return;
+  }
+  if (threadIdx.x == 0) {
+    __stcg(part + blockIdx.x, t);
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  acc = low = 0.0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += MP_THREADS) two_sum(acc, low, __ldcg(part + b), 0.0);
+  t = block_sum2<MP_THREADS>(acc, low, sh);
+  if (threadIdx.x == 0) {
+    *out = t;
+    *ticket = 0;  // for the next dot
+  }
 }
 
 // ---- segmented reduction of runs of equal keys (sorted input) -------------
@@ -171,15 +220,23 @@ int dot_impl(Ctx& c, const Vec& x, const Vec& y, double* out) {
     *out = 0.0;
     return SFCI_OK;
   }
-  u64 n = x.len + y.len;
-  u64 threads = (n + MP_ITEMS - 1) / MP_ITEMS;
-  u64 grid = (threads + MP_THREADS - 1) / MP_THREADS;
+  const u64 n = x.len + y.len;
+  // entries a thread: 8 in one block; 2 or 4 where 8 would not give every SM a block.
+  // Above four blocks an SM the last one's wait for its turn costs more than a launch
+  // (3,000,000 and 1,500,000 entries: 110 us, 103 with the sum launched).
+  const u64 block = (u64)MP_THREADS * 8, sms = (u64)c.sm_count;
+  const int items = n <= block || n > block / 2 * sms ? 8 : (n > block / 4 * sms ? 4 : 2);
+  const u64 grid = (n + (u64)MP_THREADS * items - 1) / ((u64)MP_THREADS * items);
   double* part = (double*)scratch_get(c, "dot_part", (grid + 1) * sizeof(double));
-  if (!part) return SFCI_ERR_NOMEM;
-  SFCI_LAUNCH(c, k_dot<KT>, (unsigned)grid, MP_THREADS, 0, (const KT*)x.keys, x.amps, x.len, (const KT*)y.keys,
-              y.amps, y.len, part);
-  int st = sum_parts(c, part, grid, part + grid);
-  if (st) return st;
+  const bool fresh = !c.scratch.count("dot_ticket");
+  unsigned* ticket = (unsigned*)scratch_get(c, "dot_ticket", sizeof(unsigned));
+  if (!part || !ticket) return SFCI_ERR_NOMEM;
+  if (fresh) SFCI_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), c.stream));
+  const auto kern = items == 8 ? k_dot<KT, 8> : items == 4 ? k_dot<KT, 4> : k_dot<KT, 2>;
+  SFCI_LAUNCH(c, kern, (unsigned)grid, MP_THREADS, 0, (const KT*)x.keys, (const double*)x.amps, x.len,
+              (const KT*)y.keys, (const double*)y.amps, y.len, part, grid <= 4 * sms ? ticket : nullptr, part + grid);
+  int st;
+  if (grid > 4 * sms && (st = sum_parts(c, part, grid, part + grid))) return st;
   return read_words(c, part + grid, sizeof(double), out);
 }
 
