@@ -15,7 +15,8 @@ e2e     = the same through the C ABI from pinned host buffers: host->device copy
           of the input, SpMSpV, device->host copy of the result, every step;
 roofline= dominant kernel of the step, algorithmic bytes per launch / its mean
           launch time (CUDA events on the library's stream), against the
-          measured HBM copy bandwidth; product_roofline = the whole product's
+          measured HBM copy bandwidth (null in the row form, whose terms never
+          reach HBM); product_roofline = the whole product's
           bytes under the materialise-once model (Nd + 2 T_conn + U)(K + 8)
           over the step time;
 parity  = the GPU product of the exact top-n slice that cpu_baseline times,
@@ -500,10 +501,15 @@ def _finish_gpu(args, rank, ws, dist, ctx, sysd, path, nd, M, NE, W, n_in, C, T_
                   "survivors_per_step": surv, "output_dets": out_len, "passes": stats["passes"],
                   "leaves": stats["leaves"], "partition_levels": levels,
                   "terms_gb_per_step": tbytes * T / 1e9},
-        "roofline": {"bound": "issue" if rows and dom == "merge" else "hbm", "kernel": kernels[dom], "phase": dom, "achieved": achieved, "peak": hbm,
-                     "unit": "GB/s", "frac": achieved / hbm, "peak_source": how, "traffic": traffic,
-                     "traffic_unit": "bytes per launch", "algorithmic_bytes_per_launch": per_launch_bytes,
-                     "launches": dl, "ms_per_launch": per_launch_ms},
+        "roofline": ({"bound": "issue and latency", "kernel": kernels[dom], "phase": dom, "achieved": None,
+                      "peak": None, "unit": None, "frac": None, "launches": dl, "ms_per_launch": per_launch_ms,
+                      "note": "no term reaches HBM; 57 to 61% of the issue slots are used at Nd = 2e4 "
+                              "(profiles/k_rows_cta_56orb_nd2e4.txt)"}
+                     if rows and dom == "merge" else
+                     {"bound": "hbm", "kernel": kernels[dom], "phase": dom, "achieved": achieved, "peak": hbm,
+                      "unit": "GB/s", "frac": achieved / hbm, "peak_source": how, "traffic": traffic,
+                      "traffic_unit": "bytes per launch", "algorithmic_bytes_per_launch": per_launch_bytes,
+                      "launches": dl, "ms_per_launch": per_launch_ms}),
         "product_roofline": {"bytes_model": "(Nd + 2*T_conn + U) * (K + 8)", "bytes_per_step": B,
                              "achieved": prod_ach, "peak": hbm, "unit": "GB/s", "frac": prod_ach / hbm,
                              "peak_source": how},

@@ -11,7 +11,7 @@
 // So the sources are grouped by alpha string, each row gets the list of groups
 // it receives from, and one CTA generates a row's terms and merges them in a
 // shared-memory hash table over the beta string: a term is a few loads, one FP64
-// multiplication and two or three shared-memory reductions, and nothing of it
+// multiplication and three to five shared-memory reductions, and nothing of it
 // reaches HBM.  (The partitioned pipeline of spmspv.cu writes each term once,
 // moves it through two partition levels and reads it again: 16 + 80 + 16 B.)
 //
@@ -60,18 +60,19 @@ constexpr int LIGHT_SLOTS = 256;
 // than 2^MID_BIN terms and for those above.  A step (one filling of the table)
 // costs a look at every group the row receives from, so large rows want large
 // tables, two CTAs an SM; small rows want many CTAs, whose barriers overlap.
-// Measured, 120,000 sources of 56 spin orbitals: 72.7 ms with these, 82 with 256
-// threads and 2^11 slots for the large rows, 108 with the small rows' size for
-// all; 68 spin orbitals (8-byte slots): 22 ms with 256 threads and 2^11 slots, 27
-// with 512 and 2^12 (one CTA an SM).  LOAD 0.45 / 0.65 / 0.85: 74 / 68.5 / 79 ms.
+// Measured, whole calls on 3,001, 20,000 and 120,000 sources of 56 spin orbitals: 3.12,
+// 13.0 and 63.7 ms with these, 3.24, 14.8 and 73.5 with 256 threads and 2^11 slots for
+// the large rows, 3.73, 17.9 and 94.9 with the small rows' size for all; 9,001 of 68
+// spin orbitals (8-byte slots): 20.9 ms with 256 threads and 2^11 slots, 23.0 with 512
+// and 2^12 (one CTA an SM).  LOAD 0.45 / 0.65 / 0.85 at 120,000: 69.9 / 63.7 / 68.5 ms.
 constexpr int MID_THREADS = 128, MID_TB = 10;
 template <int W> struct Big { static constexpr int threads = 512, tb = 12; };
 template <> struct Big<2> { static constexpr int threads = 256, tb = 11; };
 constexpr float LOAD = 0.65f;               // share of a table's slots a step aims to fill
 // terms per distinct target the first step of a unit assumes (later steps follow
 // the density seen).  With the previous product's mean (3.2 at 120,000 sources) a
-// tenth of the steps overflowed and were redone; with 2, one in two thousand (a
-// row has no more distinct targets than there are beta strings, either)
+// tenth of the first steps overflowed and were redone, 68.2 ms; with 2, one in two
+// thousand, 63.7 (a row has no more distinct targets than there are beta strings, either)
 constexpr float FIRST_DUP = 2.0f;
 constexpr int MID_BIN = 12;                // MID_MAX = 2^MID_BIN - 1 terms
 constexpr unsigned D1_PIECE = 128;         // entries of one source's doubles a warp takes at a time
@@ -818,13 +819,14 @@ __host__ __device__ inline size_t row_cta_smem(unsigned smax) {
   return row_table_bytes<typename StrOf<W>::T>(1u << TB) + rows_al16(sizeof(unsigned) * (smax + 1)) * 7;
 }
 
-// Larger rows: a CTA per unit.  Bound by instruction issue (12.5 warp instructions
-// a term at 23 of 32 lanes, 0.61e9 terms from 20,000 sources of 56 spin orbitals:
-// hash, two-word rounding, three or four 32-bit shared reductions, and the steps'
-// set-up); DRAM is idle and L2 serves the lists.  Whole calls with the result's
-// download, partitioned pipeline against this one: 120,000 sources of 56 spin
-// orbitals (3.7e9 terms) 178.5 and 63.4 ms, 3,001 sources 5.7 and 3.2 ms, 9,001 of
-// 68 spin orbitals 37.2 and 21.9 ms.  The unit's range of H is walked in steps
+// Larger rows: a CTA per unit.  Bound by instruction issue and by the latency that
+// half the warps an SM holds leave open: 10.8 warp instructions a term at 24 of 32
+// lanes (0.61e9 terms from 20,000 sources of 56 spin orbitals: hash, two-word
+// rounding, three to five 32-bit shared reductions, and the steps' set-up) take 61% of
+// the issue slots, the rest goes to waits, barriers and loads; DRAM is idle and L2
+// serves the lists.  Whole calls with the result's download, partitioned pipeline
+// against this one: 120,000 sources of 56 spin orbitals (3.7e9 terms) 178.5 and 63.4
+// ms, 3,001 sources 5.7 and 3.2 ms, 9,001 of 68 spin orbitals 37.2 and 21.8 ms.  The unit's range of H is walked in steps
 // that fill the table to LOAD; a step whose table overflows is redone at half its
 // width.
 template <int W, int DB, int NT, int TB_MAX>
