@@ -38,7 +38,6 @@ struct Side {
   const KT* keys;
   u64 n;
   int table;       // the keys are an open-addressing table: empty slots are skipped
-  int sorted;      // decline repeated keys (a sorted vector)
   unsigned* ra;    // alpha rank per key
   u64* arank;      // per rank: determinants | 1 << 32 when any, then their exclusive scan
   unsigned nG;
@@ -75,6 +74,7 @@ struct PairArgs {
   int up;               // ENERGY: power of two that brings the largest amplitude into [1, 2),
   double up2;           // and 4^up, by which the kets are multiplied
   u64 *plo, *phi;       // PROJECT: exact sums by bra index (split form)
+  u64 sum[2];           // ENERGY: *esum, on the host after the run
 };
 
 template <int W>
@@ -93,7 +93,7 @@ __global__ void k_pair_rank(Side<W> s, int na, int nb, int N, const unsigned* bi
     }
     ST a, b;
     split_key(k, a, b);
-    if (spop(a) != na || spop(b) != nb || !key_within(k, N) || (s.sorted && j && key_eq(k, s.keys[j - 1]))) {
+    if (spop(a) != na || spop(b) != nb || !key_within(k, N)) {
       bad = 1;
       continue;
     }
@@ -387,13 +387,9 @@ int run_pairs(Ctx& c, PairArgs<W>& a, u64 T, u64* links, bool* done) {
   *done = false;
   const ListsInUse in_use(c);
   int st;
-  KT k0;
-  if ((st = read_words(c, a.ket.keys, sizeof(KT), &k0))) return st;
   int na = 0, nb = 0;
-  for (int w = 0; w < W; ++w) {
-    na += popc64(kword(k0, w) & 0x5555555555555555ull);
-    nb += popc64(kword(k0, w) & 0xaaaaaaaaaaaaaaaaull);
-  }
+  bool alike = false;
+  if ((st = keys_one_spin<W>(c, a.ket.keys, a.ket.n, ENERGY, &na, &nb, &alike)) || !alike) return st;
   const int M = c.M, nva = M - na, nvb = M - nb;
   if (na < 1 || nb < 1 || nva < 1 || nvb < 1 || na > 16 || nb > 16) return SFCI_OK;
   const u64 RA = binom(M, na);
@@ -444,9 +440,10 @@ int run_pairs(Ctx& c, PairArgs<W>& a, u64 T, u64* links, bool* done) {
     return st;
   }
   SFCI_CUDA(cudaMemcpyAsync(tot, a.bra.arank + RA, 8, cudaMemcpyDeviceToDevice, c.stream));
-  SFCI_CUDA(cudaMemcpyAsync(tot + 1, a.ket.arank + RA, 8, cudaMemcpyDeviceToDevice, c.stream));
+  if (!ENERGY) SFCI_CUDA(cudaMemcpyAsync(tot + 1, a.ket.arank + RA, 8, cudaMemcpyDeviceToDevice, c.stream));
   u64 th[5], rb[6];
   if ((st = read_words(c, tot, sizeof th, th))) return st;
+  if (ENERGY) th[1] = th[0];
   if ((unsigned)th[4]) return SFCI_OK;
   if (ENERGY) {
     a.up = 1023 - (int)(th[3] >> 52);
@@ -490,8 +487,10 @@ int run_pairs(Ctx& c, PairArgs<W>& a, u64 T, u64* links, bool* done) {
   if (!b.ok) return SFCI_OK;
   SFCI_LAUNCH(c, (k_pair_nbrs<W, true>), ng, 256, 0, a, nslice);
   SFCI_LAUNCH(c, (k_pairs<W, ENERGY>), (unsigned)std::max<u64>(1, std::min<u64>((a.ket.n + 7) / 8, b.gmax)), 256, 0, a);
-  if ((st = read_words(c, tot + 4, 8, rb))) return st;
+  if ((st = read_words(c, tot + 4, 4 * 8, rb))) return st;
   if (rb[0] >> 32) return SFCI_OK;  // out of range: the general sweep reports it
+  a.sum[0] = rb[2];
+  a.sum[1] = rb[3];
   if (links) *links = nS + nD;
   *done = true;
   return SFCI_OK;
@@ -505,13 +504,10 @@ int pairs_energy(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   PairArgs<W> a{};
   a.bra.keys = a.ket.keys = keys;
   a.bra.n = a.ket.n = n;
-  a.bra.sorted = 1;
   a.amps = a.bamps = amps;
   int st = run_pairs<W, true>(c, a, 0, links, done);
   if (st || !*done) return st;
-  u64 s[2];
-  if ((st = read_words(c, a.esum, sizeof s, s))) return st;
-  *E = fx_to_double(s[0], s[1]) / a.up2;
+  *E = fx_to_double(a.sum[0], a.sum[1]) / a.up2;
   *terms = n * det_terms(a.na, a.nva, a.nb, c.M - a.nb);
   return SFCI_OK;
 }

@@ -49,6 +49,57 @@ __global__ void k_rows_mark(u64* __restrict__ arank, unsigned RA) {
   }
 }
 
+// out[0]: 1 where a key is not like the first (left alone otherwise); out[1..]: the first
+template <class KT>
+__global__ void k_keys_check(const KT* __restrict__ keys, u64 n, int N, int unique, u64* __restrict__ out) {
+  const KT k0 = keys[0];
+  bool bad = false;
+  for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (u64)gridDim.x * blockDim.x) {
+    const KT k = keys[j];
+    int da = 0, db = 0;
+#pragma unroll
+    for (int w = 0; w < (int)(sizeof(KT) / 8); ++w) {
+      da += popc64(kword(k, w) & 0x5555555555555555ull) - popc64(kword(k0, w) & 0x5555555555555555ull);
+      db += popc64(kword(k, w) & 0xaaaaaaaaaaaaaaaaull) - popc64(kword(k0, w) & 0xaaaaaaaaaaaaaaaaull);
+    }
+    bad |= da || db || !key_within(k, N) || (unique && j && key_eq(k, keys[j - 1]));
+  }
+  if (bad) out[0] = 1;
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(KT) / 8) out[1 + threadIdx.x] = kword(k0, threadIdx.x);
+}
+
+template <int W>
+int keys_one_spin(Ctx& c, const typename KeyOf<W>::T* keys, u64 n, bool unique, int* na, int* nb, bool* ok) {
+  const bool fresh = !c.scratch.count("keys_check");
+  u64* out = (u64*)scratch_get(c, "keys_check", 3 * 8);
+  if (!out) return SFCI_ERR_NOMEM;
+  if (fresh) SFCI_CUDA(cudaMemsetAsync(out, 0, 8, c.stream));
+  const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>((n + 255) / 256, (u64)c.sm_count * 8));
+  SFCI_LAUNCH(c, k_keys_check<typename KeyOf<W>::T>, grid, 256, 0, keys, n, c.N, unique ? 1 : 0, out);
+  u64 h[3] = {1, 0, 0};
+  int st;
+  if ((st = read_words(c, out, (1 + W) * 8, h))) return st;
+  if (h[0]) SFCI_CUDA(cudaMemsetAsync(out, 0, 8, c.stream));
+  *ok = !h[0];
+  *na = *nb = 0;
+  for (int w = 0; w < W; ++w) {
+    *na += popc64(h[1 + w] & 0x5555555555555555ull);
+    *nb += popc64(h[1 + w] & 0xaaaaaaaaaaaaaaaaull);
+  }
+  return SFCI_OK;
+}
+template int keys_one_spin<1>(Ctx&, const u64*, u64, bool, int*, int*, bool*);
+template int keys_one_spin<2>(Ctx&, const K128*, u64, bool, int*, int*, bool*);
+
+// up to four spans of 32-bit words side by side, for one readback
+struct Spans {
+  const void* p[4];
+  int n[4];
+};
+__global__ void k_rows_gather(Spans s, uint32_t* __restrict__ out) {
+  for (int q = 0; q < 4; out += s.n[q++])
+    for (int i = threadIdx.x; i < s.n[q]; i += blockDim.x) out[i] = __ldcg((const uint32_t*)s.p[q] + i);
+}
 
 namespace {
 
@@ -196,23 +247,15 @@ __global__ void k_rows_sj(HamView h, double* __restrict__ sj, double* __restrict
 template <int W>
 __global__ void k_rows_split(RowArgs<W> a) {
   typedef typename StrOf<W>::T ST;
-  unsigned bad = 0;
   for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < a.ns; j += (u64)gridDim.x * blockDim.x) {
     ST sa, sb;
     split_key(a.keys[j], sa, sb);
-    // (a repeated key would let a target receive more terms than its accumulator takes)
-    if (spop(sa) != a.na || spop(sb) != a.nb || !key_within(a.keys[j], a.h.N) ||
-        (j && key_eq(a.keys[j], a.keys[j - 1]))) {
-      bad = 1;
-      continue;
-    }
     const unsigned ra = rank_of(a.bin, sa), rb = rank_of(a.bin, sb);
     a.ra[j] = ra;
     a.rb[j] = rb;
     atomicAdd((unsigned*)(a.arank + ra), 1u);  // the low word: at most 2^31 sources
     a.brank[rb] = 1u;
   }
-  if (bad) atomicOr(a.flag, 1u);
 }
 
 // extra sources: each adds one term to the row of its own alpha string (counts,
@@ -1252,14 +1295,13 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   *done = false;
   const ListsInUse in_use(c);
   int st;
-  // spin counts of the first source (every other one is checked against them)
-  KT k0;
-  if ((st = read_words(c, keys, sizeof(KT), &k0))) return st;
+  // (a repeated key would let a target receive more terms than its accumulator takes).
+  // Other keys are declined here: with the check among the rank tables a product of
+  // 3,750 determinants of mixed spins on 14 orbitals took 90 us more, now 24, and one
+  // of two-word keys 180, now 22 (the partitioned pipeline alone 953 and 7,869).
   int na = 0, nb = 0;
-  for (int w = 0; w < W; ++w) {
-    na += popc64(kword(k0, w) & 0x5555555555555555ull);
-    nb += popc64(kword(k0, w) & 0xaaaaaaaaaaaaaaaaull);
-  }
+  bool alike = false;
+  if ((st = keys_one_spin<W>(c, keys, ns, true, &na, &nb, &alike)) || !alike) return st;
   const int M = c.M, nva = M - na, nvb = M - nb;
   if (na < 1 || nb < 1 || nva < 1 || nvb < 1 || na > ROW_EL_MAX || nb > ROW_EL_MAX) return SFCI_OK;
   const u64 RA = binom(M, na), RB = binom(M, nb);
@@ -1371,12 +1413,11 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   // the counts the host sizes the rest from
   u64* tot = (u64*)get("rw_tot", 8 * 8);
   if (!ok) return SFCI_OK;
-  SFCI_CUDA(cudaMemcpyAsync(tot, a.arank + RA, 8, cudaMemcpyDeviceToDevice, c.stream));
-  SFCI_CUDA(cudaMemcpyAsync(tot + 1, a.brank + RB, 4, cudaMemcpyDeviceToDevice, c.stream));
-  SFCI_CUDA(cudaMemcpyAsync(tot + 2, a.flag, 16, cudaMemcpyDeviceToDevice, c.stream));
   u64 th[8];
-  if ((st = read_words(c, tot, 4 * 8, th))) return st;
-  if ((unsigned)th[2]) return SFCI_OK;
+  SFCI_LAUNCH(c, k_rows_gather, 1, 64, 0, (Spans{{a.arank + RA, a.brank + RB, a.flag, nullptr}, {2, 1, 1, 0}}),
+              (uint32_t*)tot);
+  if ((st = read_words(c, tot, 2 * 8, th))) return st;
+  if (th[1] >> 32) return SFCI_OK;
   a.nG = (unsigned)(th[0] >> 32);
   a.nB = (unsigned)th[1];
   // pairs of groups and the rows they reach: 12 B each (and the same for the
@@ -1458,15 +1499,12 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
   // amortise a row's set-up
   a.unit_raw = std::max<u64>(8192, std::min<u64>(1ull << 19, T / ((u64)c.sm_count * 32)));
   SFCI_LAUNCH(c, (k_rows_units<W, false>), grid_of(RA, 2048), 256, 0, a);
-  SFCI_CUDA(cudaMemcpyAsync(tot, a.goff + a.nG, 8, cudaMemcpyDeviceToDevice, c.stream));
-  SFCI_CUDA(cudaMemcpyAsync(tot + 1, a.flag, 16, cudaMemcpyDeviceToDevice, c.stream));
+  u64* rb = (u64*)get("rw_tot2", 64 * 8);
+  if (!ok) return SFCI_OK;
   unsigned bh[64];
   {
-    u64* rb = (u64*)get("rw_tot2", 64 * 8);
-    if (!ok) return SFCI_OK;
-    SFCI_CUDA(cudaMemcpyAsync(rb, tot, 3 * 8, cudaMemcpyDeviceToDevice, c.stream));
-    SFCI_CUDA(cudaMemcpyAsync(rb + 3, a.bins, 64 * 4, cudaMemcpyDeviceToDevice, c.stream));
     u64 buf[3 + 32];
+    SFCI_LAUNCH(c, k_rows_gather, 1, 64, 0, (Spans{{a.goff + a.nG, a.flag, a.bins, nullptr}, {2, 4, 64, 0}}), (uint32_t*)rb);
     if ((st = read_words(c, rb, sizeof buf, buf))) return st;
     memcpy(th, buf, 3 * 8);
     memcpy(bh, buf + 3, sizeof bh);
@@ -1564,10 +1602,7 @@ int rows_product(Ctx& c, const typename KeyOf<W>::T* keys, const double* amps, u
     }
     side.join();
     // survivors, distinct, <v|Hv>, flags, redo count in one read
-    u64* rb = (u64*)scratch_get(c, "rw_tot2", 64 * 8);
-    SFCI_CUDA(cudaMemcpyAsync(rb, scount, 4 * 8, cudaMemcpyDeviceToDevice, c.stream));
-    SFCI_CUDA(cudaMemcpyAsync(rb + 4, a.flag, 16, cudaMemcpyDeviceToDevice, c.stream));
-    SFCI_CUDA(cudaMemcpyAsync(rb + 6, a.nredo, 4, cudaMemcpyDeviceToDevice, c.stream));
+    SFCI_LAUNCH(c, k_rows_gather, 1, 64, 0, (Spans{{scount, a.flag, a.nredo, nullptr}, {8, 4, 1, 0}}), (uint32_t*)rb);
     u64 buf[7];
     if ((st = read_words(c, rb, sizeof buf, buf))) return st;
     if ((unsigned)(buf[4] >> 32)) return SFCI_OK;  // a term above 2^max_exp

@@ -256,6 +256,10 @@ inline u64 binom(int n, int k) {
   return (u64)r;
 }
 
+// Electrons of each spin of n determinants (rows.cu): *ok when all have the same,
+// lie within the spin orbitals, and (unique) none repeats the one before it.
+template <int W>
+int keys_one_spin(Ctx& c, const typename KeyOf<W>::T* keys, u64 n, bool unique, int* na, int* nb, bool* ok);
 
 // per-context tables of rows.cu and pairs.cu: binomials, oriented opposite-spin
 // integrals and directed integrals of the singles (false: no memory)
